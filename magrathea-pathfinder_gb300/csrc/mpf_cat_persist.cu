@@ -192,9 +192,9 @@ constexpr unsigned long long kSlotNs = 2ull * 1000000000ull;
 template <int ORDER>
 __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanDev D, PropParams P, CatConst K)
 {
-    __shared__ double jac_sums[6 * kFastThreads];
-    __shared__ float jac_terms[12 * kFastThreads];
-    const JacSums J{jac_sums + threadIdx.x, jac_terms + threadIdx.x};
+    __shared__ double slot_d[kSlotDoubles * kFastThreads];
+    __shared__ float slot_f[kSlotFloats * kFastThreads];
+    const RaySlots J{slot_d + threadIdx.x, slot_f + threadIdx.x};
     const int lane = threadIdx.x & 31;
     const PropOut O{D.steps, nullptr, D.rec, D.status, nullptr};
     unsigned long long* const ctl = D.ctl;

@@ -36,10 +36,13 @@ struct DevTree {
     //   ints 0..26  the 27 cells of the cell's level around it, x-major
     //               (ix outer, iz inner), each the reference lookup result
     //               (deepest existing cell <= that level, or -1)
-    //   int 27      level | has_children << 8
+    //   int 27      node index of the cell
     //   int 28      bit j set: entry j is at exactly the cell's level
-    //   int 29      node index of the cell
+    //   int 29      level | has_children << 8 | levels up to int 31's cell << 16
     //   int 30      the parent cell (one level up), or -1
+    //   int 31      the ancestor whose stencil a TSC gather in the cell ends at
+    //               (the cell itself when all 27 entries are at its level), -1
+    //               when the gather is empty, -2 when a parent on the way is missing
     const int4* stencil;
     // per-cell velocity (vx, vy, vz, 0), or null: an octree without a
     // velocity field (the reference built without -DVELOCITYFIELD)

@@ -6,10 +6,11 @@
 //
 //  * Stencil records.  Every cell carries, in HBM, its 27 same-level
 //    neighbours resolved with the reference's lookup semantics, a mask of the
-//    ones at exactly its level and its level / children flags (built on the
-//    GPU at upload, mpf_octree.cu).  A TSC or CIC gather is then one 128-byte
-//    record load plus the payload loads; a restart at a coarser neighbour
-//    (simplehyperoctree.h:1532-1537) re-centres on the coarser cell's record.
+//    ones at exactly its level, its level / children flags and the cell whose
+//    stencil a TSC gather ends at after the restarts at coarser neighbours
+//    (simplehyperoctree.h:1532-1537; built on the GPU at upload,
+//    mpf_octree.cu).  A TSC or CIC gather is then one or two 128-byte record
+//    loads plus the payload loads.
 //    The deepest cell of a point near a known cell is read from that cell's
 //    record, so the RK stages, the post-step gather and the six Jacobian
 //    gathers of a step do no octree walks in the common case.
@@ -34,15 +35,6 @@ constexpr unsigned kFullMask = (1u << 27) - 1u;
 #endif
 #ifndef MPF_FAST_MINB
 #define MPF_FAST_MINB 2
-#endif
-// Jacobian gathers unrolled per loop trip (1: one at a time)
-#ifndef MPF_JAC_UNROLL
-#define MPF_JAC_UNROLL 1
-#endif
-constexpr int kJacUnroll = MPF_JAC_UNROLL;
-// TSC record gathers: 1 = a loop over the three x-slabs, 0 = fully unrolled
-#ifndef MPF_TSC_SLAB
-#define MPF_TSC_SLAB 0
 #endif
 constexpr int kFastThreads = MPF_FAST_THREADS;
 
@@ -115,18 +107,11 @@ __device__ __forceinline__ void point_cell(int L, double x, double y, double z, 
     }
 }
 
-__device__ __forceinline__ int rec_flags(const DevTree& T, int cell) { return __ldg(&T.stencil[8 * (size_t)cell + 6].w); }
+// level | has_children << 8 of a cell
+__device__ __forceinline__ int rec_flags(const DevTree& T, int cell) { return __ldg(&T.stencil[8 * (size_t)cell + 7].y) & 511; }
 __device__ __forceinline__ int rec_entry(const DevTree& T, int cell, int j)
 {
     return __ldg(reinterpret_cast<const int*>(T.stencil + 8 * (size_t)cell) + j);
-}
-
-// stats slots
-enum { ST_RK_REC = 0, ST_RK_SLOW, ST_POST_REC, ST_POST_SLOW, ST_JAC_REC, ST_JAC_SLOW, ST_CELL_CHANGE, ST_STEPS, ST_N };
-
-__device__ __forceinline__ void stat(unsigned long long* st, int k)
-{
-    if (st) atomicAdd(st + k, 1ull);
 }
 
 // Build-time diagnostics (-DMPF_DIAG=1): counts of the rare paths, read by
@@ -164,26 +149,22 @@ struct PosAt {
     __device__ __forceinline__ double pz() const { return z; }
 };
 
-// An RK stage point, b + c k: its float64 coordinates are formed only where a
-// rare path (a full walk, a restart at a coarser cell) needs them; the common
-// path works on the FP32 offset from the step's start cell.
-struct PosStage {
-    double bx, by, bz, dlL;
-    float cfr, kx, ky, kz;   // converted to float64 on the rare paths only
-    __device__ __forceinline__ double c() const { return (double)cfr * dlL; }
-    __device__ __forceinline__ double px() const { return fma(c(), (double)kx, bx); }
-    __device__ __forceinline__ double py() const { return fma(c(), (double)ky, by); }
-    __device__ __forceinline__ double pz() const { return fma(c(), (double)kz, bz); }
-};
-
-// A located point: its deepest cell, that cell's level, integer coordinates
-// and centre, and the point's offset from the centre in cell units.
-struct Loc {
+// A located point: its deepest cell, that cell's level and integer
+// coordinates, and the point's offset from the cell's centre in cell units.
+struct Spot {
     int cell;
     int level;
     uint32_t c[3];
+    float f[3];
+};
+// with the cell's centre
+struct Loc : Spot {
     double cen[3];
-    float fd[3];
+    __device__ __forceinline__ void centre()
+    {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) cen[d] = coord_center(level, c[d]);
+    }
 };
 
 __device__ __forceinline__ float cells_per_unit(int L) { return __int_as_float((127 + L - kLevelShift) << 23); }
@@ -197,8 +178,8 @@ static __device__ __noinline__ Loc locate_full(const DevTree& T, double x, doubl
     r.cell = f.cell;
     r.level = f.level;
     if (f.cell >= 0) {
-        point_cell(f.level, x, y, z, r.c, r.fd);
-        for (int d = 0; d < 3; ++d) r.cen[d] = coord_center(f.level, r.c[d]);
+        point_cell(f.level, x, y, z, r.c, r.f);
+        r.centre();
     }
     return r;
 }
@@ -211,10 +192,10 @@ static __device__ __noinline__ Loc locate_full(const DevTree& T, double x, doubl
 // navigated through the node array and the offsets carried in FP32, instead
 // of a float64 walk from the top grid; r.cell = -2 when neither case applies
 // (a wrapped key, a partly refined node) and the caller walks.
-static __device__ __noinline__ Loc neighbour_other(const DevTree& T, const Loc& h, int e, int fl, int ox, int oy, int oz,
-                                            float fx, float fy, float fz)
+static __device__ __noinline__ Spot neighbour_other(const DevTree& T, const Spot& h, int e, int fl, int ox, int oy, int oz,
+                                             float fx, float fy, float fz)
 {
-    Loc r;
+    Spot r;
     r.cell = -2;
     const int L = h.level;
     const int le = fl & 255;
@@ -222,13 +203,10 @@ static __device__ __noinline__ Loc neighbour_other(const DevTree& T, const Loc& 
     const uint32_t nc[3] = {h.c[0] + (uint32_t)ox, h.c[1] + (uint32_t)oy, h.c[2] + (uint32_t)oz};
     if (nc[0] > lim || nc[1] > lim || nc[2] > lim) return r;
     if (le == L && (fl & 256)) {
-        const double w = cell_extent(L);
-        double cen[3] = {h.cen[0] + (ox > 0 ? w : (ox < 0 ? -w : 0.0)), h.cen[1] + (oy > 0 ? w : (oy < 0 ? -w : 0.0)),
-                         h.cen[2] + (oz > 0 ? w : (oz < 0 ? -w : 0.0))};
         uint32_t c[3] = {nc[0], nc[1], nc[2]};
         float f[3] = {fx, fy, fz};
         int cell = e, lev = L;
-        int nd = __ldg(&T.stencil[8 * (size_t)e + 7].y);
+        int nd = __ldg(&T.stencil[8 * (size_t)e + 6].w);
         for (int guard = 0; guard < kMaxLevel; ++guard) {
             const int2 node = __ldg(T.node + nd);
             if (node.x < 0) break;   // e's descendant containing the point is a leaf
@@ -236,10 +214,8 @@ static __device__ __noinline__ Loc neighbour_other(const DevTree& T, const Loc& 
             const int nd2 = node.x + (b[0] | (b[1] << 1) | (b[2] << 2));
             const int2 child = __ldg(T.node + nd2);
             if (child.y < 0) return r;
-            const double q = pow2(kLevelShift - lev - 2);   // half the child's size
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                cen[d] += b[d] ? q : -q;
                 c[d] = 2u * c[d] + (uint32_t)b[d];
                 f[d] = 2.f * f[d] + 0.5f - (float)b[d];
             }
@@ -250,7 +226,7 @@ static __device__ __noinline__ Loc neighbour_other(const DevTree& T, const Loc& 
         r.cell = cell;
         r.level = lev;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) { r.c[d] = c[d]; r.cen[d] = cen[d]; r.fd[d] = f[d]; }
+        for (int d = 0; d < 3; ++d) { r.c[d] = c[d]; r.f[d] = f[d]; }
         return r;
     }
     if (le < L && !(fl & 256)) {
@@ -261,8 +237,7 @@ static __device__ __noinline__ Loc neighbour_other(const DevTree& T, const Loc& 
         for (int d = 0; d < 3; ++d) {
             r.c[d] = nc[d] >> k;
             const uint32_t low = nc[d] - (r.c[d] << k);
-            r.fd[d] = ((float)low + 0.5f + fn[d]) * sk - 0.5f;
-            r.cen[d] = coord_center(le, r.c[d]);
+            r.f[d] = ((float)low + 0.5f + fn[d]) * sk - 0.5f;
         }
         r.cell = e;
         r.level = le;
@@ -301,7 +276,7 @@ __device__ __forceinline__ Loc locate_rel(const DevTree& T, const Loc& h, float 
         const int ox = (int)floorf(rx + 0.5f), oy = (int)floorf(ry + 0.5f), oz = (int)floorf(rz + 0.5f);
         if (ox == 0 && oy == 0 && oz == 0) {
             Loc r = h;
-            r.fd[0] = rx; r.fd[1] = ry; r.fd[2] = rz;
+            r.f[0] = rx; r.f[1] = ry; r.f[2] = rz;
             return r;
         }
         if (abs(ox) <= 1 && abs(oy) <= 1 && abs(oz) <= 1) {
@@ -318,11 +293,15 @@ __device__ __forceinline__ Loc locate_rel(const DevTree& T, const Loc& h, float 
                     r.cen[0] = h.cen[0] + (ox > 0 ? w : (ox < 0 ? -w : 0.0));
                     r.cen[1] = h.cen[1] + (oy > 0 ? w : (oy < 0 ? -w : 0.0));
                     r.cen[2] = h.cen[2] + (oz > 0 ? w : (oz < 0 ? -w : 0.0));
-                    r.fd[0] = rx - (float)ox; r.fd[1] = ry - (float)oy; r.fd[2] = rz - (float)oz;
+                    r.f[0] = rx - (float)ox; r.f[1] = ry - (float)oy; r.f[2] = rz - (float)oz;
                     return r;
                 }
-                const Loc r = neighbour_other(T, h, e, fl, ox, oy, oz, rx - (float)ox, ry - (float)oy, rz - (float)oz);
-                if (r.cell != -2) return r;
+                Loc r;
+                static_cast<Spot&>(r) = neighbour_other(T, h, e, fl, ox, oy, oz, rx - (float)ox, ry - (float)oy, rz - (float)oz);
+                if (r.cell != -2) {
+                    r.centre();
+                    return r;
+                }
             }
         }
     }
@@ -342,40 +321,15 @@ __device__ __forceinline__ Loc locate_near(const DevTree& T, const Loc& h, doubl
     return locate_rel(T, h, rx, ry, rz, PosAt{x, y, z});
 }
 
-// The point one cell away from a located point along an axis: same in-cell
-// offset, neighbouring cell from the record (the six Jacobian points).
-__device__ __forceinline__ Loc step_cell(const DevTree& T, const Loc& h, int axis, int sgn, double x, double y, double z)
-{
-    const int ox = axis == 0 ? sgn : 0, oy = axis == 1 ? sgn : 0, oz = axis == 2 ? sgn : 0;
-    const int e = rec_entry(T, h.cell, (ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
-    if (e >= 0) {
-        const int fl = rec_flags(T, e);
-        if (!(fl & 256) && (fl & 255) == h.level) {
-            Loc r = h;
-            r.cell = e;
-            const double sw = (sgn > 0) ? cell_extent(h.level) : -cell_extent(h.level);
-            r.c[0] += ox; r.c[1] += oy; r.c[2] += oz;
-            const double moved = ((axis == 0) ? h.cen[0] : (axis == 1) ? h.cen[1] : h.cen[2]) + sw;
-            if (axis == 0) r.cen[0] = moved;
-            else if (axis == 1) r.cen[1] = moved;
-            else r.cen[2] = moved;
-            return r;
-        }
-        const Loc r = neighbour_other(T, h, e, fl, ox, oy, oz, h.fd[0], h.fd[1], h.fd[2]);
-        if (r.cell != -2) return r;
-    }
-    return locate_full(T, x, y, z);
-}
-
 // TSC at a point whose deepest cell is `cell` (simplehyperoctree.h:1479-1541
 // through the stencil records).  Returns false when a restart centre is not
 // itself a cell (left to the slow path).
 // VEL: also the velocity slots into vv[3] (with need_all).
 template <bool VEL, class P>
-__device__ __forceinline__ bool tsc_rec(const DevTree& T, const Loc& d, const P& pos, bool need_all, Field7& res, float* vv)
+__device__ __forceinline__ bool tsc_rec(const DevTree& T, const Spot& d, const P& pos, bool need_all, Field7& res, float* vv)
 {
     int cell = d.cell, L = d.level;
-    float fd[3] = {d.fd[0], d.fd[1], d.fd[2]};
+    float fd[3] = {d.f[0], d.f[1], d.f[2]};
     uint32_t c[3] = {d.c[0], d.c[1], d.c[2]};
     for (int guard = 0; guard <= kMaxLevel; ++guard) {
         const int4* rp = T.stencil + 8 * (size_t)cell;
@@ -388,30 +342,6 @@ __device__ __forceinline__ bool tsc_rec(const DevTree& T, const Loc& d, const P&
             tsc_w3(fd[2], wz);
             float gx = 0.f, gy = 0.f, gz = 0.f, gt = 0.f, rho = 0.f, phi = 0.f, a = 0.f;
             float ux = 0.f, uy = 0.f, uz = 0.f;
-#if MPF_TSC_SLAB
-            // one x-slab of 9 cells per loop trip: a third of the code of the
-            // fully unrolled loop (the kernel is instruction-fetch bound)
-            const int* re = reinterpret_cast<const int*>(rp);
-#pragma unroll 1
-            for (int ix = 0; ix < 3; ++ix) {
-                const float wxi = (ix == 0) ? wx[0] : ((ix == 1) ? wx[1] : wx[2]);
-#pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    const int e = __ldg(re + 9 * ix + k);
-                    const float wt = wxi * wy[k / 3] * wz[k % 3];
-                    const float4 g = __ldg(T.grad + e);
-                    gx = fmaf(g.x, wt, gx); gy = fmaf(g.y, wt, gy); gz = fmaf(g.z, wt, gz); gt = fmaf(g.w, wt, gt);
-                    if (need_all) {
-                        const float4 s = __ldg(T.scal + e);
-                        rho = fmaf(s.x, wt, rho); phi = fmaf(s.y, wt, phi); a = fmaf(s.z, wt, a);
-                        if (VEL) {
-                            const float4 u = __ldg(T.vel + e);
-                            ux = fmaf(u.x, wt, ux); uy = fmaf(u.y, wt, uy); uz = fmaf(u.z, wt, uz);
-                        }
-                    }
-                }
-            }
-#else
             int e[28];
 #pragma unroll
             for (int q = 0; q < 7; ++q) {
@@ -433,7 +363,6 @@ __device__ __forceinline__ bool tsc_rec(const DevTree& T, const Loc& d, const P&
                     }
                 }
             }
-#endif
             res = Field7{rho, phi, gx, gy, gz, a, gt};
             if (VEL) { vv[0] = ux; vv[1] = uy; vv[2] = uz; }
             return true;
@@ -467,10 +396,10 @@ __device__ __forceinline__ bool tsc_rec(const DevTree& T, const Loc& d, const P&
 
 // CIC at a point whose deepest cell is `cell` (simplehyperoctree.h:1410-1469).
 template <bool VEL, class P>
-__device__ __forceinline__ bool cic_rec(const DevTree& T, const Loc& d, const P& pos, bool need_all, Field7& res, float* vv)
+__device__ __forceinline__ bool cic_rec(const DevTree& T, const Spot& d, const P& pos, bool need_all, Field7& res, float* vv)
 {
     int cell = d.cell, L = d.level;
-    float fd[3] = {d.fd[0], d.fd[1], d.fd[2]};
+    float fd[3] = {d.f[0], d.f[1], d.f[2]};
     uint32_t c[3] = {d.c[0], d.c[1], d.c[2]};
     for (int guard = 0; guard <= kMaxLevel; ++guard) {
         const int sx = (fd[0] >= 0.f) ? 1 : -1, sy = (fd[1] >= 0.f) ? 1 : -1, sz = (fd[2] >= 0.f) ? 1 : -1;
@@ -529,25 +458,20 @@ __device__ __forceinline__ bool cic_rec(const DevTree& T, const Loc& d, const P&
 // where the reference's TSC falls back to CIC (simplehyperoctree.h:1570-1571)
 // VEL (with need_all): the velocity slots into vv[3] as well.
 template <int ORDER, bool VEL = false, class P>
-__device__ __forceinline__ Field7 gather_at(const DevTree& T, const Loc& d, const P& pos, bool need_all,
-                                            unsigned long long* st, int slot, bool maybe_origin, float* vv = nullptr)
+__device__ __forceinline__ Field7 gather_at(const DevTree& T, const Spot& d, const P& pos, bool need_all,
+                                            bool maybe_origin, float* vv = nullptr)
 {
     constexpr int order = ORDER;
     Field7 r;
     if (d.cell < 0) {
         clear(r);
         if (VEL) vv[0] = vv[1] = vv[2] = 0.f;
-        stat(st, slot);
         return r;
     }
     if (!(maybe_origin && pos.px() == 0.0 && pos.py() == 0.0 && pos.pz() == 0.0)) {
         const bool ok = (order == 1) ? cic_rec<VEL>(T, d, pos, need_all, r, vv) : tsc_rec<VEL>(T, d, pos, need_all, r, vv);
-        if (ok) {
-            stat(st, slot);
-            return r;
-        }
+        if (ok) return r;
     }
-    stat(st, slot + 1);
     if (VEL && need_all) return vel_slow(T, order, pos.px(), pos.py(), pos.pz(), vv);
     return (order == 1) ? cic_slow(T, pos.px(), pos.py(), pos.pz(), need_all)
                         : tsc_slow(T, pos.px(), pos.py(), pos.pz(), need_all);
@@ -628,27 +552,302 @@ __device__ __forceinline__ Rec fast_record(const FastRec& b, float data_dt, doub
     return r;
 }
 
-// Jacobian terms (d1d1, d1d2, d2d2 of lensing.h:430-447) at a trajectory
-// point located at `here`: six TSC gathers at +-1 cell.
-__device__ __forceinline__ void jac_fast(const DevTree& T, const Loc& here, double x, double y, double z, float* out3,
-                                         unsigned long long* st)
+// ---------------------------------------------------------------------------
+// Gathers of the propagation kernel.
+//
+// A gather runs in three phases that all lanes of a warp pass through
+// together: the point's cell is found, the stencil that the reference's
+// restarts end at is looked up (the record's int 31, resolved at upload), and
+// the 27 (8) cells are summed.  With the sum inside the restart loop, as the
+// point gathers above have it, a warp whose rays sit in cells of two or three
+// levels issues the sum once per level: 18.7 of 32 lanes were active per
+// instruction on a refined cone, and an RK step took 277 warp instructions
+// per photon-step.
+//
+// What bounds them is the latency of one warp's instruction stream (the 8
+// warps of an SM hide little of it), so the sums use the packed FP32 FMA
+// (fma.rn.f32x2): two fields per instruction, each rounded as fmaf rounds it.
+// Measured on refined cones (TSC, Jacobian, 60 000 rays): 282 ms -> 205 ms to
+// z = 2, 197 ms -> 141 ms for the maps of 60 000 pixels to z = 1.
+// ---------------------------------------------------------------------------
+typedef unsigned long long pair32;   // two floats in a 64-bit register
+
+__device__ __forceinline__ pair32 pack2(float a, float b)
 {
-    // dl = 2^-(level - 1 - log2 EXTENT) (lensing.h:430); h = dl / 2 = one cell of the point's level
-    const double h = pow2(kLevelShift - here.level);
-    float g[6][3];
-#pragma unroll kJacUnroll
-    for (int a = 0; a < 6; ++a) {
-        const int ax = a >> 1;
-        const int sgn = (a & 1) ? 1 : -1;
-        const double moved = ((ax == 0) ? x : (ax == 1) ? y : z) + ((a & 1) ? h : -h);
-        const double qx = (ax == 0) ? moved : x, qy = (ax == 1) ? moved : y, qz = (ax == 2) ? moved : z;
-        const Loc d = step_cell(T, here, ax, sgn, qx, qy, qz);
-        const Field7 f = gather_at<2>(T, d, PosAt{qx, qy, qz}, false, st, ST_JAC_REC, false);
-        g[a][0] = f.dx; g[a][1] = f.dy; g[a][2] = f.dz;
+    pair32 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(pair32 v, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b)
+{
+    pair32 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair32 fma2(pair32 a, pair32 b, pair32 c)
+{
+    pair32 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// An RK stage point, b + c k, and a Jacobian point: their float64 coordinates
+// are formed only where a rare path needs them.
+struct PosStage {
+    double bx, by, bz, dlL;
+    float cfr, kx, ky, kz;
+    __device__ __forceinline__ double c() const { return (double)cfr * dlL; }
+    __device__ __forceinline__ double px() const { return fma(c(), (double)kx, bx); }
+    __device__ __forceinline__ double py() const { return fma(c(), (double)ky, by); }
+    __device__ __forceinline__ double pz() const { return fma(c(), (double)kz, bz); }
+};
+struct PosShift {
+    double x, y, z;
+    int level, axis, sgn;
+    __device__ __forceinline__ double at(double v, int a) const
+    {
+        const double h = pow2(kLevelShift - level);
+        return (axis == a) ? v + (sgn > 0 ? h : -h) : v;
     }
+    __device__ __forceinline__ double px() const { return at(x, 0); }
+    __device__ __forceinline__ double py() const { return at(y, 1); }
+    __device__ __forceinline__ double pz() const { return at(z, 2); }
+};
+
+enum { kSpotSame = 0, kSpotLeaf = 1, kSpotOther = 2 };
+
+// The deepest cell of a point whose offset from the located cell h is
+// (ox, oy, oz) cells plus f (from that neighbour's centre).  r7: the last
+// quarter of the cell's record.  Returns how it was reached.
+template <class P>
+__device__ __forceinline__ int find_spot(const DevTree& T, const Spot& h, int ox, int oy, int oz, float fx, float fy, float fz,
+                                         const P& pos, Spot& d, int4& r7)
+{
+    d = h;
+    d.f[0] = fx; d.f[1] = fy; d.f[2] = fz;
+    const bool same = h.cell >= 0 && (ox | oy | oz) == 0;
+    int q = same ? h.cell : -1, kind = same ? kSpotSame : kSpotLeaf;
+    if (!same && h.cell >= 0 && abs(ox) <= 1 && abs(oy) <= 1 && abs(oz) <= 1)
+        q = rec_entry(T, h.cell, (ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
+    if (q >= 0) {
+        r7 = __ldg(T.stencil + 8 * (size_t)q + 7);
+        if (!same) {
+            const int fl = r7.y & 511;
+            if (fl == h.level) {   // a leaf of h's level
+                d.cell = q;
+                d.c[0] += (uint32_t)ox; d.c[1] += (uint32_t)oy; d.c[2] += (uint32_t)oz;
+            } else {
+                const Spot r = neighbour_other(T, h, q, fl, ox, oy, oz, fx, fy, fz);
+                kind = kSpotOther;
+                q = r.cell;
+                if (q >= 0) {
+                    d = r;
+                    r7 = __ldg(T.stencil + 8 * (size_t)q + 7);
+                }
+            }
+        }
+    }
+    if (q < 0) {
+        const Loc l = locate_full(T, pos.px(), pos.py(), pos.pz());
+        kind = kSpotOther;
+        d.cell = l.cell;
+        d.level = l.level;
+        if (l.cell >= 0) {
+#pragma unroll
+            for (int q2 = 0; q2 < 3; ++q2) { d.c[q2] = l.c[q2]; d.f[q2] = l.f[q2]; }
+            r7 = __ldg(T.stencil + 8 * (size_t)l.cell + 7);
+        }
+    }
+    return kind;
+}
+
+// The point gather through the chain of restarts, out of line: at a ray's
+// start, and for the cells whose restart the upload could not resolve.
+template <int ORDER, bool VEL>
+static __device__ __noinline__ Field7 gather_chain(const DevTree& T, const Spot& s, double x, double y, double z, int need_all,
+                                                   int maybe_origin, float* vv)
+{
+    return gather_at<ORDER, VEL>(T, s, PosAt{x, y, z}, need_all != 0, maybe_origin != 0, vv);
+}
+
+// Sum over the N cells e of a stencil with weights w(j): the gradient and
+// dphidt, with need_all the other fields, with VEL the velocity.  One chain
+// per field in the order of the cells.
+template <int N, bool VEL, class W>
+__device__ __forceinline__ void sum_cells(const DevTree& T, const int* e, const W& w, bool need_all, Field7& r, float* vv)
+{
+    pair32 gxy = 0, gzt = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const pair32 wt = w(j);
+        const ulonglong2 g = __ldg(reinterpret_cast<const ulonglong2*>(T.grad) + e[j]);
+        gxy = fma2(g.x, wt, gxy);
+        gzt = fma2(g.y, wt, gzt);
+    }
+    unpack2(gxy, r.dx, r.dy);
+    unpack2(gzt, r.dz, r.dt);
+    if (need_all) {
+        pair32 rp = 0, al = 0;   // (rho, phi), (a, the level's bits: not used)
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const pair32 wt = w(j);
+            const ulonglong2 s = __ldg(reinterpret_cast<const ulonglong2*>(T.scal) + e[j]);
+            rp = fma2(s.x, wt, rp);
+            al = fma2(s.y, wt, al);
+        }
+        float level;
+        unpack2(rp, r.rho, r.phi);
+        unpack2(al, r.a, level);
+        if (VEL) {
+            pair32 uxy = 0, uz = 0;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const pair32 wt = w(j);
+                const ulonglong2 u = __ldg(reinterpret_cast<const ulonglong2*>(T.vel) + e[j]);
+                uxy = fma2(u.x, wt, uxy);
+                uz = fma2(u.y, wt, uz);
+            }
+            float none;
+            unpack2(uxy, vv[0], vv[1]);
+            unpack2(uz, vv[2], none);
+        }
+    }
+}
+
+// TSC (ORDER 2, simplehyperoctree.h:1479-1541) or CIC (ORDER 1, :1410-1469) at
+// a located point; r7: the last quarter of its cell's record.
+template <int ORDER, bool VEL, class P>
+__device__ __forceinline__ Field7 gather_spot(const DevTree& T, const Spot& d, const int4& r7, const P& pos, bool need_all,
+                                              float* vv)
+{
+    Field7 r;
+    clear(r);
+    if (VEL) vv[0] = vv[1] = vv[2] = 0.f;
+    int cell = d.cell, state = (cell >= 0) ? 0 : -1;   // 0: sum, -1: empty, -2: through the chain of restarts
+    float fd[3] = {d.f[0], d.f[1], d.f[2]};
+    if (ORDER == 2) {
+        if (cell >= 0) {
+            const int t = r7.w;
+            int k = r7.y >> 16;
+            if (t >= 0) {
+                cell = t;
+                uint32_t c[3] = {d.c[0], d.c[1], d.c[2]};
+                for (; k > 0; --k) {   // the point's offset in its ancestor, one level at a time
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        fd[q] = (fd[q] + (float)(c[q] & 1u) - 0.5f) * 0.5f;
+                        c[q] >>= 1;
+                    }
+                }
+            } else {
+                state = t;
+            }
+        }
+        if (state == 0) {
+            const int4* rp = T.stencil + 8 * (size_t)cell;
+            int e[28];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const int4 v = __ldg(rp + q);
+                e[4 * q] = v.x; e[4 * q + 1] = v.y; e[4 * q + 2] = v.z; e[4 * q + 3] = v.w;
+            }
+            float wx[3], wy[3], wz[3];
+            tsc_w3(fd[0], wx);
+            tsc_w3(fd[1], wy);
+            tsc_w3(fd[2], wz);
+            pair32 w2[9], wx2[3];   // wy * wz is shared by the three x-slabs
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const float v = wy[q / 3] * wz[q % 3];
+                w2[q] = pack2(v, v);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) wx2[q] = pack2(wx[q], wx[q]);
+            sum_cells<27, VEL>(T, e, [&](int j) { return mul2(wx2[j / 9], w2[j % 9]); }, need_all, r, vv);
+        }
+    } else {
+        // the eight cells of the point's octant: entries s0 + {0, 1} x 9 + {0, 1} x 3 + {0, 1}
+        constexpr unsigned kOct = 0x1u | 0x2u | 0x8u | 0x10u | 0x200u | 0x400u | 0x1000u | 0x2000u;
+        int s0 = 0;
+        if (cell >= 0) {
+            int L = d.level;
+            unsigned exact = (unsigned)r7.x;
+            uint32_t c[3] = {d.c[0], d.c[1], d.c[2]};
+            for (int guard = 0;; ++guard) {
+                s0 = ((fd[0] >= 0.f) ? 9 : 0) + ((fd[1] >= 0.f) ? 3 : 0) + ((fd[2] >= 0.f) ? 1 : 0);
+                if (((exact >> s0) & kOct) == kOct) break;
+                // a coarser or a missing one: again on the ancestor at the coarsest of the eight's levels
+                int lvl = L;
+                for (int v = 0; v < 8; ++v) {
+                    const int e = rec_entry(T, cell, s0 + 9 * (v & 1) + 3 * ((v >> 1) & 1) + (v >> 2));
+                    if (e < 0) break;
+                    lvl = min(lvl, rec_flags(T, e) & 255);
+                }
+                if (lvl == L) { state = -1; break; }
+                cell = ancestor_up(T, cell, L, lvl, c, fd);
+                if (cell < 0 || guard >= kMaxLevel) { state = -2; break; }
+                L = lvl;
+                exact = (unsigned)__ldg(&T.stencil[8 * (size_t)cell + 7].x);
+            }
+        }
+        if (state == 0) {
+            int e[8];
+#pragma unroll
+            for (int v = 0; v < 8; ++v) e[v] = rec_entry(T, cell, s0 + 9 * (v & 1) + 3 * ((v >> 1) & 1) + (v >> 2));
+            // the neighbour on the point's side gets |fd|, the centre cell 1 - |fd| (per axis)
+            float w0[3], w1[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float a = fabsf(fd[q]);
+                w0[q] = (fd[q] >= 0.f) ? 1.f - a : a;
+                w1[q] = (fd[q] >= 0.f) ? a : 1.f - a;
+            }
+            sum_cells<8, VEL>(T, e, [&](int v) {
+                const float w = ((v & 1) ? w1[0] : w0[0]) * ((v & 2) ? w1[1] : w0[1]) * ((v & 4) ? w1[2] : w0[2]);
+                return pack2(w, w);
+            }, need_all, r, vv);
+        }
+    }
+    if (state == -2) r = gather_chain<ORDER, VEL>(T, d, pos.px(), pos.py(), pos.pz(), need_all, 0, vv);
+    return r;
+}
+
+// Jacobian terms (d1d1, d1d2, d2d2 of lensing.h:430-447) at a trajectory
+// point located at `here`: six TSC gathers at +-1 cell of the point's level,
+// the same in-cell offset in the neighbouring cell of the record.
+__device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, double x, double y, double z, float* out3)
+{
+    // differences of the plus and minus points, before 1 / dl
+    float dxx = 0.f, dxy = 0.f, dxz = 0.f, dyy = 0.f, dyz = 0.f, dzz = 0.f;
+#pragma unroll 1
+    for (int axis = 0; axis < 3; ++axis) {
+        float mx = 0.f, my = 0.f, mz = 0.f;
+#pragma unroll 1
+        for (int sgn = -1; sgn <= 1; sgn += 2) {
+            const int ox = axis == 0 ? sgn : 0, oy = axis == 1 ? sgn : 0, oz = axis == 2 ? sgn : 0;
+            const PosShift pos{x, y, z, here.level, axis, sgn};
+            Spot d;
+            int4 r7;
+            find_spot(T, here, ox, oy, oz, here.f[0], here.f[1], here.f[2], pos, d, r7);
+            const Field7 f = gather_spot<2, false>(T, d, r7, pos, false, nullptr);
+            if (sgn < 0) {
+                mx = f.dx; my = f.dy; mz = f.dz;
+            } else if (axis == 0) {
+                dxx = f.dx - mx;
+            } else if (axis == 1) {
+                dxy = f.dx - mx; dyy = f.dy - my;
+            } else {
+                dxz = f.dx - mx; dyz = f.dy - my; dzz = f.dz - mz;
+            }
+        }
+    }
+    // dl = 2^-(level - 1 - log2 EXTENT) (lensing.h:430), twice the shift
     const float idl = __int_as_float((127 + here.level - kLevelShift - 1) << 23);   // 1 / dl, exact
-    const float dxx = (g[1][0] - g[0][0]) * idl, dxy = (g[3][0] - g[2][0]) * idl, dxz = (g[5][0] - g[4][0]) * idl;
-    const float dyy = (g[3][1] - g[2][1]) * idl, dyz = (g[5][1] - g[4][1]) * idl, dzz = (g[5][2] - g[4][2]) * idl;
+    dxx *= idl; dxy *= idl; dxz *= idl; dyy *= idl; dyz *= idl; dzz *= idl;
     const float fx = (float)x, fy = (float)y, fz = (float)z;
     const float rho = sqrtf(fx * fx + fy * fy);
     const float r = sqrtf(fx * fx + fy * fy + fz * fz);
@@ -661,17 +860,37 @@ __device__ __forceinline__ void jac_fast(const DevTree& T, const Loc& here, doub
               cp * s2t * dxz;
 }
 
-// Per-thread Jacobian running sums kept in shared memory (touched once per
-// step, so they need not occupy registers through the gathers): the FP64
-// sums S (6), and the last point's contribution c_k (6) and the one before it
-// c_km1 (6), FP32 products of the point's FP32 Hessian terms; strided by the
-// block size.
-struct JacSums {
-    double* sums;   // this thread's slot 0 of S
-    float* terms;   // this thread's slot 0 of c_k, c_km1
-    __device__ __forceinline__ double& S(int q) const { return sums[q * kFastThreads]; }
-    __device__ __forceinline__ float& ck(int q) const { return terms[q * kFastThreads]; }
-    __device__ __forceinline__ float& ckm1(int q) const { return terms[(6 + q) * kFastThreads]; }
+// Per-thread values that a step touches once, kept in shared memory so that
+// they do not occupy registers through the gathers; strided by the block
+// size.  S: the Jacobian's FP64 running sums; ck, ckm1: the last point's
+// contribution to them and the one before it (FP32 products of the point's
+// FP32 Hessian terms); cen: the centre of the point's cell; the running
+// integrals of the ray; the comoving distances of the last two points before
+// the current one; the last step's length and change of phi.
+constexpr int kSlotDoubles = 16;
+constexpr int kSlotFloats = 14;
+struct RaySlots {
+    double* d;
+    float* f;
+    __device__ __forceinline__ double& S(int q) const { return d[q * kFastThreads]; }
+    __device__ __forceinline__ double& cen(int q) const { return d[(6 + q) * kFastThreads]; }
+    __device__ __forceinline__ double& lambda() const { return d[9 * kFastThreads]; }
+    __device__ __forceinline__ double& s() const { return d[10 * kFastThreads]; }
+    __device__ __forceinline__ double& isw() const { return d[11 * kFastThreads]; }
+    __device__ __forceinline__ double& iswold() const { return d[12 * kFastThreads]; }
+    __device__ __forceinline__ double& chim1() const { return d[13 * kFastThreads]; }
+    __device__ __forceinline__ double& chim2() const { return d[14 * kFastThreads]; }
+    __device__ __forceinline__ double& last_dl() const { return d[15 * kFastThreads]; }
+    __device__ __forceinline__ float& ck(int q) const { return f[q * kFastThreads]; }
+    __device__ __forceinline__ float& ckm1(int q) const { return f[(6 + q) * kFastThreads]; }
+    __device__ __forceinline__ float& last_dphi() const { return f[12 * kFastThreads]; }
+    __device__ __forceinline__ float& rmax() const { return f[13 * kFastThreads]; }
+};
+
+// a trajectory point's state and the field there
+struct RayPoint {
+    double a, t, x, y, z, k0, k1, k2, k3, chi;
+    Field7 g;
 };
 
 // SRC: source mode (one surface at the ray's own radius); WIDE: per-ray
@@ -683,7 +902,7 @@ struct JacSums {
 // (integrator.h:707-708, 765-767); plain instantiations only.
 template <int ORDER, bool SRC, bool WIDE, bool BORN = false, bool VEL = false>
 __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropParams& P, const double* L, long long i,
-                               const PropOut& O, JacSums J)
+                               const PropOut& O, RaySlots J)
 {
     const double c2 = kC * kC;
     const double mn = -(double)kExtent / 2.0, mx = (double)kExtent / 2.0;
@@ -694,7 +913,6 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     const double* rpl = (WIDE && P.ray_planes) ? P.ray_planes + i * np : P.planes;   // this ray's surfaces
     const double stop_ref = SRC ? P.ray_stop[i] : ((WIDE && P.ray_planes) ? rpl[np - 1] : P.stop_ref);
     const int rec_fields = SRC ? kSourceFields : (WIDE ? kWideFields : kPlaneFields);
-    unsigned long long* const st = O.stats;
     // Born ray (Order = -1 on the octree itself: hmaps.h:706-712,
     // catalogues.h:670-673), an instantiation of its own: the homogeneous
     // field in the stages and after each step, the octree's levels for the
@@ -703,73 +921,51 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     Field7 hom;
     clear(hom);
     hom.a = 1.f;
-    FastRec b;
+    RayPoint b;
+    b.a = 1.0; b.t = 0.0; b.x = L[0]; b.y = L[1]; b.z = L[2]; b.k0 = 1.0;
     if (SRC || (WIDE && P.direct)) {
         // (phi, theta) launch form or a bundle photon: the direction is given
-        b.a = 1.0; b.t = 0.0; b.x = L[0]; b.y = L[1]; b.z = L[2]; b.k0 = 1.0;
         b.k1 = L[3]; b.k2 = L[4]; b.k3 = L[5];
     } else {
-        const double norm = sqrt((L[3] - L[0]) * (L[3] - L[0]) + (L[4] - L[1]) * (L[4] - L[1]) + (L[5] - L[2]) * (L[5] - L[2]));
-        b.a = 1.0; b.t = 0.0; b.x = L[0]; b.y = L[1]; b.z = L[2]; b.k0 = 1.0;
-        b.k1 = (L[3] - L[0]) / norm; b.k2 = (L[4] - L[1]) / norm; b.k3 = (L[5] - L[2]) / norm;
+        const double A = L[3] - L[0], B = L[4] - L[1], D = L[5] - L[2];
+        const double norm = sqrt(A * A + B * B + D * D);
+        b.k1 = A / norm; b.k2 = B / norm; b.k3 = D / norm;
     }
-    Loc here = locate_full(T, b.x, b.y, b.z);
+    Spot here;
     float vv[3] = {0.f, 0.f, 0.f};   // VEL: the velocity of the last post-step gather
-    Field7 data = born ? hom : gather_at<ORDER, VEL>(T, here, PosAt{b.x, b.y, b.z}, true, st, ST_POST_REC, true, vv);
     {
-        const double ph = (double)data.phi / c2;
+        const Loc l = locate_full(T, b.x, b.y, b.z);
+        here = l;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) J.cen(a) = l.cen[a];
+        b.g = born ? hom : gather_chain<ORDER, VEL>(T, l, b.x, b.y, b.z, 1, 1, vv);
+    }
+    {
+        const double ph = (double)b.g.phi / c2;
         const double norm = sqrt((c2 * (1.0 + 2.0 * ph) * b.k0 * b.k0) / ((1.0 - 2.0 * ph) * (b.k1 * b.k1 + b.k2 * b.k2 + b.k3 * b.k3)));
         b.k1 *= norm; b.k2 *= norm; b.k3 *= norm;
     }
     const double v0n = VEL ? (P.vobs[0] * b.k1 + P.vobs[1] * b.k2 + P.vobs[2] * b.k3) / (kC * b.k0) : 0.0;
-    b.dop = 0.0;
+    double bdop = 0.0;
     // data != empty (integrator.h:715): with VEL the velocity slots count too
-    auto empty = [&]() -> bool { return is_empty(data) && (!VEL || (vv[0] == 0.f && vv[1] == 0.f && vv[2] == 0.f)); };
+    auto empty = [&](const Field7& f) -> bool { return is_empty(f) && (!VEL || (vv[0] == 0.f && vv[1] == 0.f && vv[2] == 0.f)); };
     b.a = interp_fast(C, b.t, C.a, C.slope_a);
-    b.level = (here.cell >= 0) ? here.level : 0;
-    b.ah = 0.f;
-    b.rho = data.rho; b.phi = data.phi; b.dx = data.dx; b.dy = data.dy; b.dz = data.dz; b.dt = data.dt;
-    b.red = 0.0; b.isw = 0.0; b.chi = 0.0; b.iswold = 0.0; b.lambda = 0.0; b.s = 0.0;
+    float bdt = b.g.dt;   // the photon's (forward) dphidt
+    float bah = 0.f;
+    b.chi = 0.0;
     const double ratio_k = (scale / kC) / P.nsteps;
-    double ratio = b.a * b.a * ratio_k;
-    double dl = (here.cell >= 0 ? cell_extent(here.level) : 0.0) * ratio;
+    double dl = (here.cell >= 0 ? cell_extent(here.level) : 0.0) * (b.a * b.a * ratio_k);
     const double a0 = b.a;
     int tb = bracket_lut(C, b.t);       // cosmology-table bracket of the ray's conformal time
-    const double phi0c2 = b.phi / c2;
-    float last_data_dt = data.dt;
-    float last_dphi = 0.f;
-    double last_dl = 1.0;
-
-    // every trajectory point (bundle rays), wide instantiation only
-    double* const traj = (WIDE && O.traj) ? O.traj + i * O.traj_cap * kPhotonFields : nullptr;
-    if (WIDE && traj && O.traj_cap > 0) write_rec(traj, fast_record(b, 0.f, 0.0, 0));
-    int next_plane = 0;
-    long long cross_k[kMaxPlanes];
-    for (int j = 0; j < np; ++j) cross_k[j] = -1;
-    double* prow = O.plane_rec ? O.plane_rec + (long long)i * np * rec_fields : nullptr;
-    if (SRC && prow) {
-        prow[24] = b.a; prow[25] = b.phi; prow[26] = b.k1; prow[27] = b.k2; prow[28] = b.k3;
-        prow[29] = prow[30] = prow[31] = 0.0;
-    }
-    // this ray's plane normals (stop criterion "plane" with per-ray surfaces; wide instantiation)
-    const double* rki = (WIDE && P.ray_ki) ? P.ray_ki + i * np * 3 : nullptr;
-    auto start_q = [&](int jn) -> double {
-        if (rki && skind == STOP_PLANE) return b.x * rki[3 * jn] + b.y * rki[3 * jn + 1] + b.z * rki[3 * jn + 2];
-        return (skind == STOP_R) ? b.chi : (skind == STOP_LAMBDA) ? b.lambda : (skind == STOP_T) ? b.t
-             : (skind == STOP_S) ? b.s : b.red;
-    };
-    while (next_plane < np && ((skind == STOP_A) ? (b.a < (SRC ? stop_ref : rpl[next_plane]))
-                                                  : (start_q(next_plane) > (SRC ? stop_ref : rpl[next_plane])))) {
-        cross_k[next_plane] = 0;
-        ++next_plane;
-    }
-    double rmax = 0.0;
-    bool have_rmax = false;
+    const double phi0c2 = (double)b.g.phi / c2;
     for (int q = 0; q < 6; ++q) { J.S(q) = 0.0; J.ck(q) = 0.f; J.ckm1(q) = 0.f; }
-    double chim1 = 0.0, chim2 = 0.0;
+    J.chim1() = J.chim2() = 0.0;
+    J.isw() = J.iswold() = J.lambda() = J.s() = 0.0;
+    J.last_dl() = 1.0;
+    J.last_dphi() = 0.f;
+    J.rmax() = 0.f;
     long long k = 0;
     unsigned status = 0;
-    double isw = 0.0, iswold = 0.0, lambda = 0.0, sacc = 0.0;
     // A point's redshift (integrator.h:769) is formed only where it is read:
     // surface records, the end of the ray, trajectory records.  The stop and
     // crossing tests compare a0 (1 + phi0/c^2 - phi/c^2) with (1 + z) a
@@ -777,17 +973,51 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     const double opc = 1.0 + phi0c2;
     const double inv_c2 = 1.0 / c2;
     // VEL: a0 / a (1 + phi0/c^2 - phi/c^2 + isw + v.k / (c k0) - v0n) - 1
-    auto zbracket = [&](const FastRec& r) -> double {
-        if (VEL) return opc - r.phi * inv_c2 + r.isw + r.dop - v0n;
-        return opc - r.phi * inv_c2;
+    auto zbracket = [&](float phi, double isw, double dop) -> double {
+        if (VEL) return opc - (double)phi * inv_c2 + isw + dop - v0n;
+        return opc - (double)phi * inv_c2;
     };
-    auto red_of = [&](const FastRec& r) -> double { return a0 * recip(r.a) * zbracket(r) - 1.0; };
-    auto red_above = [&](const FastRec& r, double zref) -> bool { return a0 * zbracket(r) > (1.0 + zref) * r.a; };
-    bool b_red_ok = true;     // b.red holds b's redshift
+    auto red_of = [&](double a, float phi, double isw, double dop) -> double { return a0 * recip(a) * zbracket(phi, isw, dop) - 1.0; };
+    auto red_above = [&](double a, float phi, double isw, double dop, double zref) -> bool {
+        return a0 * zbracket(phi, isw, dop) > (1.0 + zref) * a;
+    };
+    // the point b as the reference's photon record
+    auto full_point = [&]() -> FastRec {
+        FastRec r;
+        r.a = b.a; r.t = b.t; r.x = b.x; r.y = b.y; r.z = b.z; r.k0 = b.k0; r.k1 = b.k1; r.k2 = b.k2; r.k3 = b.k3;
+        r.phi = b.g.phi; r.chi = b.chi; r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw(); r.iswold = J.iswold();
+        r.red = (k == 0) ? 0.0 : red_of(b.a, b.g.phi, r.isw, bdop);
+        r.rho = b.g.rho; r.dx = b.g.dx; r.dy = b.g.dy; r.dz = b.g.dz; r.dt = bdt; r.ah = bah;
+        r.level = (here.cell >= 0) ? here.level : 0;
+        return r;
+    };
+
+    // every trajectory point (bundle rays), wide instantiation only
+    double* const traj = (WIDE && O.traj) ? O.traj + i * O.traj_cap * kPhotonFields : nullptr;
+    if (WIDE && traj && O.traj_cap > 0) write_rec(traj, fast_record(full_point(), 0.f, 0.0, 0));
+    int next_plane = 0;
+    long long cross_k[kMaxPlanes];
+    for (int j = 0; j < np; ++j) cross_k[j] = -1;
+    double* prow = O.plane_rec ? O.plane_rec + (long long)i * np * rec_fields : nullptr;
+    if (SRC && prow) {
+        prow[24] = b.a; prow[25] = b.g.phi; prow[26] = b.k1; prow[27] = b.k2; prow[28] = b.k3;
+        prow[29] = prow[30] = prow[31] = 0.0;
+    }
+    // this ray's plane normals (stop criterion "plane" with per-ray surfaces; wide instantiation)
+    const double* rki = (WIDE && P.ray_ki) ? P.ray_ki + i * np * 3 : nullptr;
+    auto start_q = [&](int jn) -> double {
+        if (rki && skind == STOP_PLANE) return b.x * rki[3 * jn] + b.y * rki[3 * jn + 1] + b.z * rki[3 * jn + 2];
+        return (skind == STOP_T) ? b.t : 0.0;   // chi, lambda, s and the redshift start at 0
+    };
+    while (next_plane < np && ((skind == STOP_A) ? (b.a < (SRC ? stop_ref : rpl[next_plane]))
+                                                  : (start_q(next_plane) > (SRC ? stop_ref : rpl[next_plane])))) {
+        cross_k[next_plane] = 0;
+        ++next_plane;
+    }
     const float two_c2 = (float)(2.0 / c2);
     const float inv_c2f = (float)(1.0 / c2);
-    FastRec p;
-    while (!empty()) {
+    bool go = !empty(b.g);
+    while (go) {
         if (k >= P.max_steps) { status |= 1u; break; }
         // ---- RK4 step (integrator.h:718-734).  The state stays FP64 and is
         // accumulated in FP64; the four stages are evaluated in FP32 as
@@ -859,250 +1089,281 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         // terms of k (E), the stage increments (S) and the a' terms (SA)
         float Gd = 0.f, Gk = 0.f, Se = 0.f, E0 = 0.f, E1 = 0.f, E2 = 0.f, E3 = 0.f;
         float S0 = 0.f, S1 = 0.f, S2 = 0.f, S3 = 0.f, SA = 0.f;
-        float dtf;   // the step's conformal-time increment
+        float dtf = 0.f, ds = 0.f;   // the step's conformal-time increment and path length
+        RayPoint p;
+        Spot q;
+        int kind = kSpotSame;
+        Field7 g = b.g;
+        // stages 1-4, then the post-step point: stage 1 is at b, where the
+        // previous step's post-step gather read the field; stages 2-4 are
+        // located from their FP32 offset to b's cell, the post-step point from
+        // its float64 offset
 #pragma unroll 1
-        for (int sg = 0; sg < 4; ++sg) {
+        for (int sg = 0; sg < 5; ++sg) {
             const float cfr = (sg == 0) ? 0.f : ((sg < 3) ? 0.5f : 1.f);
-            const float w = (sg == 0 || sg == 3) ? 1.f : 2.f;
-            const float cdl = cfr * dlf;
-            const float q0 = cdl * d0, q1 = cdl * d1, q2 = cdl * d2, q3 = cdl * d3;
-            const float k0 = kb0 + q0, k1 = kb1 + q1, k2 = kb2 + q2, k3 = kb3 + q3;
-            const float as = fmaf(cdl, dA, abf);
-            const float dad = dadot(cdl * pk0);
-            // stage 1 is at b, where the previous step's post-step gather read
-            // the field (data); stages 2-4 are located from their FP32 offset
-            // to b's cell, their float64 coordinates formed only on the rare
-            // full-walk / restart paths
-            Field7 g = data;
-            if (sg > 0) {
-                g = hom;
-                if (!born) {
-                    const float cc = cfr * dlLf * cpu;
-                    const PosStage ps{b.x, b.y, b.z, dlL, cfr, pk1, pk2, pk3};
-                    const Loc d = locate_rel(T, here, fmaf(cc, pk1, here.fd[0]), fmaf(cc, pk2, here.fd[1]),
-                                             fmaf(cc, pk3, here.fd[2]), ps);
-                    g = gather_at<ORDER>(T, d, ps, false, st, ST_RK_REC, false);
-                }
+            if (sg == 4) {
+                const double dl6 = dl * (1.0 / 6.0), dlL6 = dlL * (1.0 / 6.0);
+                const float dl6f = (float)dl6, dlL6f = (float)dlL6;
+                const double h6 = hubb * (6.0 + (double)Se);
+                const double cd = dl6 * ((double)Gd - h6);
+                p.k0 = fma(b.k0, dl6 * (-h6 - (double)Gk), b.k0 + (double)(dl6f * E0));
+                p.k1 = fma(b.k1, cd, b.k1 + (double)(dl6f * E1));
+                p.k2 = fma(b.k2, cd, b.k2 + (double)(dl6f * E2));
+                p.k3 = fma(b.k3, cd, b.k3 + (double)(dl6f * E3));
+                p.x = fma(dlL, b.k1, b.x + (double)(dlL6f * S1));
+                p.y = fma(dlL, b.k2, b.y + (double)(dlL6f * S2));
+                p.z = fma(dlL, b.k3, b.z + (double)(dlL6f * S3));
+                p.t = fma(dl, b.k0, b.t + (double)(dl6f * S0));
+                const double da = __dmul_rn(dl * b.k0, adb);
+                p.a = fma(da, (double)(SA * (1.f / 6.f)), __dadd_rn(b.a, da));
+                // the step's displacement and conformal-time increment in FP32
+                // (path length s and the ISW integral)
+                const float ex = fmaf(dlLf, kb1, dlL6f * S1), ey = fmaf(dlLf, kb2, dlL6f * S2), ez = fmaf(dlLf, kb3, dlL6f * S3);
+                ds = sqrtf(ex * ex + ey * ey + ez * ez);
+                dtf = fmaf(dlf, kb0, dl6f * S0);
             }
-            const float gk = g.dx * k1 + (g.dy * k2 + g.dz * k3);
-            const float dphidl = fmaf(g.dt, k0, gk);
-            // the drag at the stage relative to b: a' (1 + u), a / (1 - v'), k0 (1 + wk)
-            const float u = dad * inv_adbf, v = -(cdl * dA) / as, wk = q0 * inv_kb0;
-            const float eps = u + v + wk + (u * v + u * wk + v * wk) + u * v * wk;
-            const float hub = hubbf * (1.f + eps);
-            const float coef = two_c2 * dphidl - hub;
-            const float coef0 = -hub - two_c2 * gk;
-            const float k02 = 2.f * k0 * k0;
-            const float G1 = g.dx * k02, G2 = g.dy * k02, G3 = g.dz * k02;
-            Gd = fmaf(w, two_c2 * dphidl, Gd);
-            Gk = fmaf(w, two_c2 * gk, Gk);
-            Se = fmaf(w, eps, Se);
-            E0 = fmaf(w, coef0 * q0, E0);
-            E1 = fmaf(w, fmaf(coef, q1, -G1), E1);
-            E2 = fmaf(w, fmaf(coef, q2, -G2), E2);
-            E3 = fmaf(w, fmaf(coef, q3, -G3), E3);
-            S0 = fmaf(w, q0, S0); S1 = fmaf(w, q1, S1); S2 = fmaf(w, q2, S2); S3 = fmaf(w, q3, S3);
-            SA = fmaf(w, u + wk + u * wk, SA);
-            d0 = coef0 * k0;
-            d1 = fmaf(coef, k1, -G1); d2 = fmaf(coef, k2, -G2); d3 = fmaf(coef, k3, -G3);
-            dA = k0 * (adbf + dad);
-            pk0 = k0; pk1 = k1; pk2 = k2; pk3 = k3;
+            if (sg > 0 && (!born || sg == 4)) {
+                float rx, ry, rz;
+                if (sg == 4) {
+                    rx = (float)(p.x - J.cen(0)) * cpu; ry = (float)(p.y - J.cen(1)) * cpu; rz = (float)(p.z - J.cen(2)) * cpu;
+                } else {
+                    const float cc = cfr * dlLf * cpu;
+                    rx = fmaf(cc, pk1, here.f[0]); ry = fmaf(cc, pk2, here.f[1]); rz = fmaf(cc, pk3, here.f[2]);
+                }
+                // the post-step point's own coordinates stand in for the stage form (c = 0)
+                const PosStage ps = (sg == 4) ? PosStage{p.x, p.y, p.z, 0.0, 0.f, 0.f, 0.f, 0.f}
+                                              : PosStage{b.x, b.y, b.z, dlL, cfr, pk1, pk2, pk3};
+                const int ox = (int)floorf(rx + 0.5f), oy = (int)floorf(ry + 0.5f), oz = (int)floorf(rz + 0.5f);
+                int4 r7;
+                kind = find_spot(T, here, ox, oy, oz, rx - (float)ox, ry - (float)oy, rz - (float)oz, ps, q, r7);
+                if (!born) g = gather_spot<ORDER, VEL>(T, q, r7, ps, sg == 4, vv);
+            }
+            if (sg < 4) {
+                if (born && sg > 0) g = hom;
+                const float cdl = cfr * dlf;
+                const float q0 = __fmul_rn(cdl, d0), q1 = __fmul_rn(cdl, d1), q2 = __fmul_rn(cdl, d2), q3 = __fmul_rn(cdl, d3);
+                const float w = (sg == 0 || sg == 3) ? 1.f : 2.f;
+                const float k0 = kb0 + q0, k1 = kb1 + q1, k2 = kb2 + q2, k3 = kb3 + q3;
+                const float as = fmaf(cdl, dA, abf);
+                const float dad = dadot(cdl * pk0);
+                // (the products that are contracted are written out here and below:
+                // every instantiation then rounds a step alike)
+                const float gk = fmaf(g.dx, k1, fmaf(g.dz, k3, __fmul_rn(g.dy, k2)));
+                const float dphidl = fmaf(g.dt, k0, gk);
+                // the drag at the stage relative to b: a' (1 + u), a / (1 - v'), k0 (1 + wk)
+                const float u = dad * inv_adbf, v = -(cdl * dA) / as, wk = q0 * inv_kb0;
+                const float uv = __fmul_rn(u, v);
+                const float eps = fmaf(uv, wk, (u + v + wk) + fmaf(v, wk, fmaf(u, wk, uv)));
+                // 2 / c^2 times a sum, less the drag hubb (1 + eps)
+                const float tg = __fmul_rn(two_c2, dphidl), tk = __fmul_rn(two_c2, gk);
+                const float coef = fmaf(-hubbf, 1.f + eps, tg);
+                const float coef0 = fmaf(-hubbf, 1.f + eps, -tk);
+                const float k02 = 2.f * k0 * k0;
+                const float G1 = g.dx * k02, G2 = g.dy * k02, G3 = g.dz * k02;
+                Gd = fmaf(w, tg, Gd);
+                Gk = fmaf(w, tk, Gk);
+                Se = fmaf(w, eps, Se);
+                E0 = fmaf(w, coef0 * q0, E0);
+                E1 = fmaf(w, fmaf(coef, q1, -G1), E1);
+                E2 = fmaf(w, fmaf(coef, q2, -G2), E2);
+                E3 = fmaf(w, fmaf(coef, q3, -G3), E3);
+                S0 = fmaf(w, q0, S0); S1 = fmaf(w, q1, S1); S2 = fmaf(w, q2, S2); S3 = fmaf(w, q3, S3);
+                SA = fmaf(w, fmaf(u, wk, u + wk), SA);
+                d0 = coef0 * k0;
+                d1 = fmaf(coef, k1, -G1); d2 = fmaf(coef, k2, -G2); d3 = fmaf(coef, k3, -G3);
+                dA = k0 * (adbf + dad);
+                pk0 = k0; pk1 = k1; pk2 = k2; pk3 = k3;
+            }
         }
-        {
-            const double dl6 = dl * (1.0 / 6.0), dlL6 = dlL * (1.0 / 6.0);
-            const float dl6f = (float)dl6, dlL6f = (float)dlL6;
-            const double h6 = hubb * (6.0 + (double)Se);
-            const double cd = dl6 * ((double)Gd - h6);
-            p.k0 = fma(b.k0, dl6 * (-h6 - (double)Gk), b.k0 + (double)(dl6f * E0));
-            p.k1 = fma(b.k1, cd, b.k1 + (double)(dl6f * E1));
-            p.k2 = fma(b.k2, cd, b.k2 + (double)(dl6f * E2));
-            p.k3 = fma(b.k3, cd, b.k3 + (double)(dl6f * E3));
-            p.x = fma(dlL, b.k1, b.x + (double)(dlL6f * S1));
-            p.y = fma(dlL, b.k2, b.y + (double)(dlL6f * S2));
-            p.z = fma(dlL, b.k3, b.z + (double)(dlL6f * S3));
-            p.t = fma(dl, b.k0, b.t + (double)(dl6f * S0));
-            const double da = dl * b.k0 * adb;
-            p.a = fma(da, (double)(SA * (1.f / 6.f)), b.a + da);
-            // the step's displacement and conformal-time increment in FP32
-            // (path length s and the ISW integral)
-            const float ex = fmaf(dlLf, kb1, dlL6f * S1), ey = fmaf(dlLf, kb2, dlL6f * S2), ez = fmaf(dlLf, kb3, dlL6f * S3);
-            sacc += (double)sqrtf(ex * ex + ey * ey + ez * ez);
-            dtf = fmaf(dlf, kb0, dl6f * S0);
-        }
-        const Loc ploc = locate_near(T, here, p.x, p.y, p.z);
-        data = born ? hom : gather_at<ORDER, VEL>(T, ploc, PosAt{p.x, p.y, p.z}, true, st, ST_POST_REC, false, vv);
+        p.g = born ? hom : g;
         {
             // the extent test (integrator.h:757): a point in a located cell away from
             // the domain faces is inside; only cells on a face (or wrapped keys)
             // need the float64 comparison
-            const uint32_t last = (ploc.cell >= 0) ? (uint32_t)((1ull << ploc.level) - 1ull) : 0u;
-            const bool face = (ploc.cell < 0) || ploc.c[0] == 0u || ploc.c[1] == 0u || ploc.c[2] == 0u ||
-                              ploc.c[0] >= last || ploc.c[1] >= last || ploc.c[2] >= last;
+            const uint32_t last = (q.cell >= 0) ? (uint32_t)((1ull << q.level) - 1ull) : 0u;
+            const bool face = (q.cell < 0) || q.c[0] == 0u || q.c[1] == 0u || q.c[2] == 0u ||
+                              q.c[0] >= last || q.c[1] >= last || q.c[2] >= last;
             if (p.a < 0.0 || (face && !((p.x > mn) && (p.x < mx) && (p.y > mn) && (p.y < mx) && (p.z > mn) && (p.z < mx)))) {
-                clear(data);
+                clear(p.g);
                 if (VEL) vv[0] = vv[1] = vv[2] = 0.f;
             }
         }
-        if (VEL) p.dop = ((double)vv[0] * p.k1 + (double)vv[1] * p.k2 + (double)vv[2] * p.k3) / (kC * p.k0);
-        p.level = (ploc.cell >= 0) ? ploc.level : 0;
-        p.ah = data.a;
-        p.rho = data.rho; p.phi = data.phi; p.dx = data.dx; p.dy = data.dy; p.dz = data.dz;
-        p.dt = -data.dt;
-        const float dphi_last = data.phi - (float)b.phi;   // laplacian of the final record, divided at the end
-        const double dl_last = dl;
-        isw += (double)((b.dt + p.dt) * dtf * inv_c2f);
-        if (O.final_rec) {   // only the final photon record reports it
-            iswold -= 2.0 * (p.phi - b.phi) * (1.0 / c2) -
-                      (((double)b.dx + (double)p.dx) * (p.x - b.x) * scale + ((double)b.dy + (double)p.dy) * (p.y - b.y) * scale +
-                       ((double)b.dz + (double)p.dz) * (p.z - b.z) * scale) * (1.0 / c2);
+        if (empty(p.g)) break;   // the new point is not appended: the ray ends at b
+        const double pdop = VEL ? ((double)vv[0] * p.k1 + (double)vv[1] * p.k2 + (double)vv[2] * p.k3) / (kC * p.k0) : 0.0;
+        const float pdt = -p.g.dt;
+        const double b_isw = J.isw(), b_s = J.s(), b_lambda = J.lambda();
+        const double p_isw = b_isw + (double)((bdt + pdt) * dtf * inv_c2f);
+        const double p_s = b_s + (double)ds;
+        const double p_lambda = b_lambda + dl;
+        J.isw() = p_isw;
+        J.s() = p_s;
+        J.lambda() = p_lambda;
+        if (O.final_rec || (WIDE && traj)) {   // reported by photon records only
+            if (O.final_rec)
+                J.iswold() -= 2.0 * ((double)p.g.phi - (double)b.g.phi) * (1.0 / c2) -
+                              (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) * scale + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) * scale +
+                               ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z) * scale) * (1.0 / c2);
+            J.last_dphi() = p.g.phi - b.g.phi;   // laplacian of the record, divided there
+            J.last_dl() = dl;
         }
         p.chi = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
-        lambda += dl;
-        p.isw = isw; p.iswold = iswold; p.lambda = lambda; p.s = sacc;
-        bool p_red_ok = false;
-        auto need_p_red = [&]() { if (!p_red_ok) { p.red = red_of(p); p_red_ok = true; } };
-        auto need_b_red = [&]() { if (!b_red_ok) { b.red = red_of(b); b_red_ok = true; } };
-        if (!empty()) {
-            const double ratio = p.a * p.a * ratio_k;
-            dl = (ploc.cell >= 0 ? cell_extent(ploc.level) : 0.0) * ratio;
-            last_data_dt = data.dt;
-            last_dphi = dphi_last;
-            last_dl = dl_last;
-            if (ploc.cell != here.cell) stat(st, ST_CELL_CHANGE);
-            here = ploc;
-            ++k;
-            stat(st, ST_STEPS);
-            if (P.jacobian) {
-                float h3[3];
-                jac_fast(T, here, p.x, p.y, p.z, h3, st);
-                const float dr = (float)(p.chi - b.chi), chif = (float)p.chi;
-                chim2 = chim1; chim1 = b.chi;
+        dl = (q.cell >= 0 ? cell_extent(q.level) : 0.0) * (p.a * p.a * ratio_k);
+        ++k;
+        // the surfaces the step crossed: everything but the Jacobian, from b and p
+        const int first_crossed = next_plane;
+        bool p_red_known = false;   // the stop test below reads p's redshift where a surface formed it
+        double p_red = 0.0;
+        while (next_plane < np) {
+            const double* kj = (WIDE && rki && skind == STOP_PLANE) ? rki + 3 * next_plane : nullptr;
+            const double ref = SRC ? stop_ref : rpl[next_plane];
+            bool crossed;
+            double q1 = 0.0;
+            if (!kj && skind == STOP_REDSHIFT) {
+                crossed = red_above(p.a, p.g.phi, p_isw, pdop, ref);
+            } else {
+                if (!kj && skind == STOP_PLANE && !p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, pdop); p_red_known = true; }
+                q1 = kj ? (p.x * kj[0] + p.y * kj[1] + p.z * kj[2])
+                   : (skind == STOP_R) ? p.chi : (skind == STOP_LAMBDA) ? p_lambda : (skind == STOP_T) ? p.t
+                   : (skind == STOP_A) ? p.a : (skind == STOP_S) ? p_s : p_red;
+                crossed = (skind == STOP_A) ? (q1 < ref) : (q1 > ref);
+            }
+            if (!crossed) break;
+            const int j = next_plane++;
+            cross_k[j] = k;
+            if (prow) {
+                if (!p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, pdop); p_red_known = true; }
+                const double b_red = (k == 1) ? 0.0 : red_of(b.a, b.g.phi, b_isw, bdop);
+                double* o = prow + j * rec_fields;
+                if (!kj && skind == STOP_REDSHIFT) q1 = p_red;
+                const double q0 = kj ? (b.x * kj[0] + b.y * kj[1] + b.z * kj[2])
+                                : (skind == STOP_R) ? b.chi : (skind == STOP_LAMBDA) ? b_lambda : (skind == STOP_T) ? b.t
+                                : (skind == STOP_A) ? b.a : (skind == STOP_S) ? b_s : b_red;
+                const double f = (q1 - ref) / (q1 - q0);
+                const double px = b.x * f + p.x * (1 - f), py = b.y * f + p.y * (1 - f), pz = b.z * f + p.z * (1 - f);
+                o[0] = (double)(k - 1); o[1] = f; o[2] = px; o[3] = py; o[4] = pz; o[5] = sqrt(px * px + py * py + pz * pz);
+                o[6] = o[7] = o[8] = 0.0;
+                o[9] = b.t * f + p.t * (1 - f);
+                o[10] = b.a * f + p.a * (1 - f);
+                o[11] = b_red * f + p_red * (1 - f);
+                o[12] = b.chi * f + p.chi * (1 - f);
+                o[13] = b_lambda * f + p_lambda * (1 - f);
+                o[14] = b_s * f + p_s * (1 - f);
+                o[15] = b_isw * f + p_isw * (1 - f);
+                o[16] = (double)b.g.rho * f + (double)p.g.rho * (1 - f);
+                o[17] = (double)b.g.phi * f + (double)p.g.phi * (1 - f);
+                o[18] = (k >= 2) ? (double)J.rmax() : 0.0;
+                o[19] = 1.0;
+                if (SRC || WIDE) {
+                    o[20] = b.k0 * f + p.k0 * (1 - f);
+                    o[21] = b.k1 * f + p.k1 * (1 - f);
+                    o[22] = b.k2 * f + p.k2 * (1 - f);
+                    o[23] = b.k3 * f + p.k3 * (1 - f);
+                }
+            }
+        }
+        // the largest density of the points before the new one
+        if (k == 1 || J.rmax() < b.g.rho) J.rmax() = b.g.rho;
+        // p becomes the ray's last point
+        const float dr = (float)(p.chi - b.chi);
+        const double chi_b = b.chi;
+        b = p;
+        bdt = pdt;
+        bah = p.g.a;
+        bdop = pdop;
+        if (kind != kSpotSame) {
+            if (kind == kSpotLeaf) {
+                // +-w or 0 per axis (selects, no int-to-double conversion)
+                const double w = cell_extent(q.level);
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    J.ckm1(q) = J.ck(q); J.ckm1(3 + q) = J.ck(3 + q);
-                    const float c1 = chif * (h3[q] * dr), c2v = chif * c1;
-                    J.ck(q) = c1;
-                    J.ck(3 + q) = c2v;
-                    J.S(q) += (double)c1;
-                    J.S(3 + q) += (double)c2v;
+                for (int a = 0; a < 3; ++a) {
+                    const int o = (int)(q.c[a] - here.c[a]);
+                    if (o != 0) J.cen(a) += (o > 0) ? w : -w;
                 }
+            } else if (q.cell >= 0) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) J.cen(a) = coord_center(q.level, q.c[a]);
             }
-            while (next_plane < np) {
-                const int kind = skind;
-                const double* kj = (WIDE && rki && kind == STOP_PLANE) ? rki + 3 * next_plane : nullptr;
-                const double ref = SRC ? stop_ref : rpl[next_plane];
-                bool crossed;
-                if (!kj && kind == STOP_REDSHIFT) {
-                    crossed = red_above(p, ref);
+        }
+        here = q;
+        if (P.jacobian) {
+            float h3[3];
+            jac_fast(T, here, b.x, b.y, b.z, h3);
+            const float chif = (float)b.chi;
+            J.chim2() = J.chim1();
+            J.chim1() = chi_b;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                J.ckm1(a) = J.ck(a); J.ckm1(3 + a) = J.ck(3 + a);
+                const float c1 = chif * (h3[a] * dr), c2v = chif * c1;
+                J.ck(a) = c1;
+                J.ck(3 + a) = c2v;
+                J.S(a) += (double)c1;
+                J.S(3 + a) += (double)c2v;
+            }
+            for (int j = first_crossed; prow && j < next_plane; ++j) {
+                // at the surface's distance, or at the source radius in source
+                // mode, or at the surface radius itself for a Born ray
+                double* o = prow + j * rec_fields;
+                const double jd = (SRC || born) ? (SRC ? stop_ref : rpl[j]) : o[5];
+                double s1[3], s2[3];
+                bool ok = true;
+                if (b.chi <= jd) {
+                    for (int a = 0; a < 3; ++a) { s1[a] = J.S(a); s2[a] = J.S(3 + a); }
+                } else if (chi_b <= jd) {
+                    for (int a = 0; a < 3; ++a) { s1[a] = J.S(a) - (double)J.ck(a); s2[a] = J.S(3 + a) - (double)J.ck(3 + a); }
+                } else if (k >= 2 && J.chim2() <= jd) {
+                    for (int a = 0; a < 3; ++a) {
+                        s1[a] = J.S(a) - (double)J.ck(a) - (double)J.ckm1(a);
+                        s2[a] = J.S(3 + a) - (double)J.ck(3 + a) - (double)J.ckm1(3 + a);
+                    }
                 } else {
-                    const double q1 = kj ? (p.x * kj[0] + p.y * kj[1] + p.z * kj[2])
-                                    : (kind == STOP_R) ? p.chi : (kind == STOP_LAMBDA) ? p.lambda : (kind == STOP_T) ? p.t
-                                    : (kind == STOP_A) ? p.a : (kind == STOP_S) ? p.s : (need_p_red(), p.red);
-                    crossed = (kind == STOP_A) ? (q1 < ref) : (q1 > ref);
+                    ok = false;
+                    status |= 2u;
                 }
-                if (!crossed) break;
-                const int j = next_plane++;
-                cross_k[j] = k;
-                if (prow) {
-                    need_p_red();
-                    need_b_red();
-                    double* o = prow + j * rec_fields;
-                    const double q1 = kj ? (p.x * kj[0] + p.y * kj[1] + p.z * kj[2])
-                                    : (kind == STOP_R) ? p.chi : (kind == STOP_LAMBDA) ? p.lambda : (kind == STOP_T) ? p.t
-                                    : (kind == STOP_A) ? p.a : (kind == STOP_S) ? p.s : p.red;
-                    const double q0 = kj ? (b.x * kj[0] + b.y * kj[1] + b.z * kj[2])
-                                    : (kind == STOP_R) ? b.chi : (kind == STOP_LAMBDA) ? b.lambda : (kind == STOP_T) ? b.t
-                                    : (kind == STOP_A) ? b.a : (kind == STOP_S) ? b.s : b.red;
-                    const double f = (q1 - ref) / (q1 - q0);
-                    const double px = b.x * f + p.x * (1 - f), py = b.y * f + p.y * (1 - f), pz = b.z * f + p.z * (1 - f);
-                    const double dist = sqrt(px * px + py * py + pz * pz);
-                    o[0] = (double)(k - 1); o[1] = f; o[2] = px; o[3] = py; o[4] = pz; o[5] = dist;
-                    o[9] = b.t * f + p.t * (1 - f);
-                    o[10] = b.a * f + p.a * (1 - f);
-                    o[11] = b.red * f + p.red * (1 - f);
-                    o[12] = b.chi * f + p.chi * (1 - f);
-                    o[13] = b.lambda * f + p.lambda * (1 - f);
-                    o[14] = b.s * f + p.s * (1 - f);
-                    o[15] = b.isw * f + p.isw * (1 - f);
-                    o[16] = (double)b.rho * f + (double)p.rho * (1 - f);
-                    o[17] = b.phi * f + p.phi * (1 - f);
-                    o[18] = have_rmax ? rmax : 0.0;
-                    o[19] = 1.0;
-                    if (SRC || WIDE) {
-                        o[20] = b.k0 * f + p.k0 * (1 - f);
-                        o[21] = b.k1 * f + p.k1 * (1 - f);
-                        o[22] = b.k2 * f + p.k2 * (1 - f);
-                        o[23] = b.k3 * f + p.k3 * (1 - f);
-                    }
-                    if (P.jacobian) {
-                        // at the surface's distance, or at the source radius in source
-                        // mode, or at the surface radius itself for a Born ray
-                        const double jd = (SRC || born) ? ref : dist;
-                        double s1[3], s2[3];
-                        bool ok = true;
-                        if (p.chi <= jd) {
-                            for (int q = 0; q < 3; ++q) { s1[q] = J.S(q); s2[q] = J.S(3 + q); }
-                        } else if (chim1 <= jd) {
-                            for (int q = 0; q < 3; ++q) { s1[q] = J.S(q) - (double)J.ck(q); s2[q] = J.S(3 + q) - (double)J.ck(3 + q); }
-                        } else if (k >= 2 && chim2 <= jd) {
-                            for (int q = 0; q < 3; ++q) {
-                                s1[q] = J.S(q) - (double)J.ck(q) - (double)J.ckm1(q);
-                                s2[q] = J.S(3 + q) - (double)J.ck(3 + q) - (double)J.ckm1(3 + q);
-                            }
-                        } else {
-                            ok = false;
-                            status |= 2u;
-                        }
-                        if (ok) {
-                            const double idist = 1.0 / jd;
-                            o[6] = 1.0 - 2.0 * (s1[0] - s2[0] * idist) / c2 * P.length;
-                            o[7] = -2.0 * (s1[1] - s2[1] * idist) / c2 * P.length;
-                            o[8] = 1.0 - 2.0 * (s1[2] - s2[2] * idist) / c2 * P.length;
-                        } else {
-                            o[6] = 1.0; o[7] = 0.0; o[8] = 1.0;
-                        }
-                    } else {
-                        o[6] = o[7] = o[8] = 0.0;
-                    }
+                if (ok) {
+                    const double idist = 1.0 / jd;
+                    o[6] = 1.0 - 2.0 * (s1[0] - s2[0] * idist) / c2 * P.length;
+                    o[7] = -2.0 * (s1[1] - s2[1] * idist) / c2 * P.length;
+                    o[8] = 1.0 - 2.0 * (s1[2] - s2[2] * idist) / c2 * P.length;
+                } else {
+                    o[6] = 1.0; o[7] = 0.0; o[8] = 1.0;
                 }
             }
-            if (!have_rmax || rmax < (double)b.rho) rmax = b.rho;
-            have_rmax = true;
-            b = p;
-            b_red_ok = p_red_ok;
-            if (WIDE && traj) {
-                need_b_red();
-                if (k < O.traj_cap) write_rec(traj + k * kPhotonFields, fast_record(b, last_data_dt, (double)last_dphi / last_dl, k));
-                else status |= 8u;
-            }
+        }
+        if (WIDE && traj) {
+            const FastRec r = full_point();
+            p_red = r.red;
+            p_red_known = true;
+            if (k < O.traj_cap) write_rec(traj + k * kPhotonFields, fast_record(r, -bdt, (double)J.last_dphi() / J.last_dl(), k));
+            else status |= 8u;
         }
         bool stop;
         switch (skind) {
         case STOP_R: stop = b.chi > stop_ref; break;
-        case STOP_LAMBDA: stop = b.lambda > stop_ref; break;
-        case STOP_REDSHIFT: stop = b_red_ok ? (b.red > stop_ref) : red_above(b, stop_ref); break;
+        case STOP_LAMBDA: stop = J.lambda() > stop_ref; break;
+        case STOP_REDSHIFT: stop = p_red_known ? (p_red > stop_ref) : red_above(b.a, b.g.phi, J.isw(), bdop, stop_ref); break;
         case STOP_T: stop = b.t > stop_ref; break;
         case STOP_A: stop = b.a < stop_ref; break;
         case STOP_PLANE: {
             const double* kk = (WIDE && rki) ? rki + 3 * (np - 1) : P.ki;
-            stop = (p.x * kk[0] + p.y * kk[1] + p.z * kk[2]) > stop_ref;
+            stop = (b.x * kk[0] + b.y * kk[1] + b.z * kk[2]) > stop_ref;
             break;
         }
-        case STOP_S: stop = b.s > stop_ref; break;
+        case STOP_S: stop = J.s() > stop_ref; break;
         default: stop = true;
         }
-        if (stop) break;
+        go = !stop;
     }
-    if (!b_red_ok) b.red = red_of(b);
+    const FastRec r = full_point();
     long long size = k + 1;
-    if (signbit(b.red) || signbit(b.a)) size -= 1;
+    if (signbit(r.red) || signbit(r.a)) size -= 1;
     O.steps[i] = size;
     if (O.final_rec) {
         double* o = O.final_rec + i * kPhotonFields;
         if (size == k + 1) {
-            write_rec(o, fast_record(b, last_data_dt, (double)last_dphi / last_dl, k));
+            write_rec(o, fast_record(r, -bdt, (double)J.last_dphi() / J.last_dl(), k));
         } else {
-            for (int q = 0; q < kPhotonFields; ++q) o[q] = 0.0;
+            for (int a = 0; a < kPhotonFields; ++a) o[a] = 0.0;
             status |= 4u;
         }
     }
@@ -1151,7 +1412,6 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     if (status) atomicOr(O.status, status);
 }
 
-
 // Persistent launch: each warp takes the next 32 x depth rays of [lo, n) from
 // a global counter until the range is exhausted, so uneven path lengths do
 // not leave tail waves; its lanes trace them depth at a time.  `queue` is
@@ -1167,9 +1427,9 @@ __global__ void MPF_FAST_BOUNDS k_propagate_fast(DevTree T, DevCosmo C, PropPara
                                                                     const double* __restrict__ launch, long long n, PropOut O,
                                                                     unsigned long long* queue, int depth, long long lo)
 {
-    __shared__ double jac_sums[6 * kFastThreads];
-    __shared__ float jac_terms[12 * kFastThreads];
-    const JacSums J{jac_sums + threadIdx.x, jac_terms + threadIdx.x};
+    __shared__ double slot_d[kSlotDoubles * kFastThreads];
+    __shared__ float slot_f[kSlotFloats * kFastThreads];
+    const RaySlots J{slot_d + threadIdx.x, slot_f + threadIdx.x};
     const int lane = threadIdx.x & 31;
     const unsigned long long per = 32ull * (unsigned long long)depth;
     for (;;) {
@@ -1196,8 +1456,8 @@ static __global__ void k_gather_rec(DevTree T, int kind, const double* __restric
         ((long long*)out)[i] = d.cell;
         return;
     }
-    const Field7 f = (kind == 1) ? gather_at<1>(T, d, PosAt{x, y, z}, true, nullptr, 0, true)
-                                 : gather_at<2>(T, d, PosAt{x, y, z}, true, nullptr, 0, true);
+    const Field7 f = (kind == 1) ? gather_at<1>(T, d, PosAt{x, y, z}, true, true)
+                                 : gather_at<2>(T, d, PosAt{x, y, z}, true, true);
     float* o = (float*)out + 7 * i;
     o[0] = f.rho; o[1] = f.phi; o[2] = f.dx; o[3] = f.dy; o[4] = f.dz; o[5] = f.a; o[6] = f.dt;
 }

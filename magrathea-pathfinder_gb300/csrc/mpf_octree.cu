@@ -206,9 +206,9 @@ __global__ void k_stencil(DevTree T, const int* cell_node, int4* out)
                 if (f.cell >= 0 && f.level == L) exact |= 1u << j;
             }
     const int nd = cell_node[i];
-    e[27] = L | ((T.node[nd].x >= 0) ? 256 : 0);
+    e[27] = nd;
     e[28] = (int)exact;
-    e[29] = nd;
+    e[29] = L | ((T.node[nd].x >= 0) ? 256 : 0);
     // the parent cell (one level up), for restarts at coarser levels
     int parent = -1;
     if (L - 1 >= T.Lt) {
@@ -216,9 +216,39 @@ __global__ void k_stencil(DevTree T, const int* cell_node, int4* out)
         if (f.cell >= 0 && f.level == L - 1) parent = f.cell;
     }
     e[30] = parent;
-    e[31] = 0;
+    e[31] = (exact == (1u << 27) - 1u) ? (int)i : -2;
     int4* o = out + 8 * i;
     for (int q = 0; q < 8; ++q) o[q] = make_int4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
+}
+
+// Where a TSC gather in a cell with a coarser or missing neighbour ends: the
+// reference starts again at the level of the first one (x-major,
+// simplehyperoctree.h:1532-1537), on the point's ancestor there, until a
+// stencil is complete or a neighbour is missing.  The chain depends on the
+// cell alone, so it is followed once here.  Only int 31 and the upper half of
+// int 29 are written, which no other thread reads.
+__global__ void k_restart(int64_t n, int4* rec)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const unsigned full = (1u << 27) - 1u;
+    int* const r = reinterpret_cast<int*>(rec);
+    unsigned exact = (unsigned)r[32 * i + 28];
+    if (exact == full) return;
+    int64_t cell = i;
+    const int L = r[32 * i + 29] & 255;
+    int l = L, target = -2;
+    for (int guard = 0; guard <= kMaxLevel; ++guard) {
+        if (exact == full) { target = (int)cell; break; }
+        const int e = r[32 * cell + __ffs(~exact & full) - 1];
+        if (e < 0) { target = -1; break; }
+        const int lc = r[32 * (int64_t)e + 29] & 255;
+        for (; l > lc && cell >= 0; --l) cell = r[32 * cell + 30];
+        if (cell < 0 || l != lc) break;
+        exact = (unsigned)r[32 * cell + 28];
+    }
+    r[32 * i + 31] = target;
+    if (target >= 0) r[32 * i + 29] |= (L - l) << 16;
 }
 
 inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -385,6 +415,7 @@ extern "C" int mpf_internal_octree_build(const void* records, int64_t n, int on_
     if (!dalloc((void**)&o->stencil, (size_t)n * 8 * sizeof(int4), false)) { release(true); return fail("out of device memory", -2); }
     o->tree.stencil = o->stencil;
     k_stencil<<<blocks(n, 128), 128, 0, stream>>>(o->tree, cell_node, o->stencil);
+    k_restart<<<blocks(n, 256), 256, 0, stream>>>(n, o->stencil);
     ce = cudaStreamSynchronize(stream);
     if (ce == cudaSuccess) ce = cudaGetLastError();
     release(false);

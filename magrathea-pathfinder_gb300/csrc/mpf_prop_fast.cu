@@ -257,10 +257,12 @@ cudaError_t launch_propagate<false>(const DevTree& T, const DevCosmo& C, const P
     long long grid = 0;
     int tpb_used = fast_launch_shape(n, st.blocks_per_sm, st.sms, &grid);
     int depth = 1;
-    // MPF_STATS=1: count record-path gathers and slow-path fallbacks (diagnostics; serialises the call)
+#if MPF_DIAG
+    // MPF_STATS=1: print the counts of the rare paths (diagnostics; serialises the call)
     static const bool want_stats = getenv("MPF_STATS") != nullptr;
+#endif
     static const bool want_tune = !(getenv("MPF_AUTOTUNE") && getenv("MPF_AUTOTUNE")[0] == '0');
-    if (tpb_used == kFastThreads && want_tune && !want_stats) {
+    if (tpb_used == kFastThreads && want_tune) {
         // a batch that fills the GPU: the tuned shape of this octree and kernel mode
         int dev = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -289,27 +291,16 @@ cudaError_t launch_propagate<false>(const DevTree& T, const DevCosmo& C, const P
             grid = shape_grid(res.best, n, st.sms);
         }
     }
-    PropOut o2 = O;
-    unsigned long long* dstats = nullptr;
-    if (want_stats && cudaMalloc(&dstats, ST_N * sizeof(unsigned long long)) == cudaSuccess) {
-        cudaMemsetAsync(dstats, 0, ST_N * sizeof(unsigned long long), stream);
-        o2.stats = dstats;
-    }
-    launch_fast_kernel(grid, tpb_used, depth, 0, T, C, P, d_launch, n, o2, queue, stream);
+    launch_fast_kernel(grid, tpb_used, depth, 0, T, C, P, d_launch, n, O, queue, stream);
     e = cudaGetLastError();
-    if (dstats) {
-        unsigned long long h[ST_N];
-        cudaMemcpyAsync(h, dstats, sizeof(h), cudaMemcpyDeviceToHost, stream);
-        cudaStreamSynchronize(stream);
-        fprintf(stderr, "mpf_stats rk_rec %llu rk_slow %llu post_rec %llu post_slow %llu jac_rec %llu jac_slow %llu cell_changes %llu steps %llu\n",
-                h[0], h[1], h[2], h[3], h[4], h[5], h[6], h[7]);
 #if MPF_DIAG
+    if (want_stats) {
         unsigned long long dg[4] = {0, 0, 0, 0};
+        cudaStreamSynchronize(stream);
         cudaMemcpyFromSymbol(dg, g_diag, sizeof(dg));
         fprintf(stderr, "mpf_diag restarts %llu full_walks %llu\n", dg[0], dg[1]);
-#endif
-        cudaFree(dstats);
     }
+#endif
     return e;
 }
 cudaError_t launch_gather_fast(const DevTree& T, int kind, const double* d_xyz, long long n, void* d_out, cudaStream_t stream)

@@ -95,7 +95,6 @@ struct PropOut {
     double* final_rec;     // n x 28, or null
     double* plane_rec;     // n x nplanes x 20, or null
     unsigned* status;      // bit 0: a ray hit max_steps
-    unsigned long long* stats;   // optional path counters (fast mode), or null
     double* traj;          // n x traj_cap x 28: every trajectory point, or null
     long long traj_cap;    // points kept per ray (status bit 3 when a ray has more)
 };

@@ -255,7 +255,7 @@ extern "C" int mpf_rays_propagate(const mpf_octree* o, const mpf_cosmology* c, c
         e = cudaMemcpy(dl.p, launch.data(), (size_t)m * nt * 6 * sizeof(double), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemset(dstatus.p, 0, sizeof(unsigned));
         if (e != cudaSuccess) return cuda_fail(e, "mpf_rays_propagate");
-        PropOut O{(long long*)dsteps.p, nullptr, nullptr, (unsigned*)dstatus.p, nullptr, (double*)dtraj.p, cap};
+        PropOut O{(long long*)dsteps.p, nullptr, nullptr, (unsigned*)dstatus.p, (double*)dtraj.p, cap};
         e = (p->exact || hom) ? launch_propagate<true>(o->tree, C, P, (const double*)dl.p, m * nt, O, 0)
                      : launch_propagate<false>(o->tree, C, P, (const double*)dl.p, m * nt, O, 0);
         unsigned hs = 0;

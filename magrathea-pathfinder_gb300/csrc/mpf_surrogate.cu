@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_propagate_surrogate(DevTree T, 
                 b.a = 1.0; b.t = 0.0; b.x = L[0]; b.y = L[1]; b.z = L[2]; b.k0 = 1.0;
                 b.k1 = (L[3] - L[0]) / norm0; b.k2 = (L[4] - L[1]) / norm0; b.k3 = (L[5] - L[2]) / norm0;
                 here = locate_full(T, b.x, b.y, b.z);
-                data = gather_at<ORDER>(T, here, PosAt{b.x, b.y, b.z}, true, nullptr, 0, true);
+                data = gather_at<ORDER>(T, here, PosAt{b.x, b.y, b.z}, true, true);
                 const double ph = (double)data.phi / c2;
                 const double nk = sqrt((c2 * (1.0 + 2.0 * ph) * b.k0 * b.k0) / ((1.0 - 2.0 * ph) * (b.k1 * b.k1 + b.k2 * b.k2 + b.k3 * b.k3)));
                 b.k1 *= nk; b.k2 *= nk; b.k3 *= nk;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_propagate_surrogate(DevTree T, 
                     ++k;
                     if (check_every > 0 && (k % check_every) == 0) {
                         // checkpoint: the octree's field at the same point
-                        const Field7 go = gather_at<ORDER>(T, here, PosAt{p.x, p.y, p.z}, false, nullptr, 0, false);
+                        const Field7 go = gather_at<ORDER>(T, here, PosAt{p.x, p.y, p.z}, false, false);
                         const double kn = rsqrt(p.k1 * p.k1 + p.k2 * p.k2 + p.k3 * p.k3);
                         const double nx = p.k1 * kn, ny = p.k2 * kn, nz = p.k3 * kn;
                         const double w = p.chi - chi_ck;
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_propagate_surrogate(DevTree T, 
         if (active && finish) {
             // final checkpoint at the last accepted point, then the drift test
             if (k > 0 && here.cell >= 0 && b.chi > chi_ck) {
-                const Field7 go = gather_at<ORDER>(T, here, PosAt{b.x, b.y, b.z}, false, nullptr, 0, false);
+                const Field7 go = gather_at<ORDER>(T, here, PosAt{b.x, b.y, b.z}, false, false);
                 const double kn = rsqrt(b.k1 * b.k1 + b.k2 * b.k2 + b.k3 * b.k3);
                 const double nx = b.k1 * kn, ny = b.k2 * kn, nz = b.k3 * kn;
                 const double w = b.chi - chi_ck;
@@ -527,7 +527,7 @@ __global__ void k_sample(DevTree T, Cone K, Spec S, uint64_t seed, const long lo
     const double py = px * K.tan_y * (2.0 * unit(h1) - 1.0);
     const double pz = px * K.tan_z * (2.0 * unit(h2) - 1.0);
     const Loc d = locate_full(T, px, py, pz);
-    const Field7 f = gather_at<2>(T, d, PosAt{px, py, pz}, true, nullptr, 0, false);
+    const Field7 f = gather_at<2>(T, d, PosAt{px, py, pz}, true, false);
     x[4 * b] = (float)px; x[4 * b + 1] = (float)py; x[4 * b + 2] = (float)pz; x[4 * b + 3] = f.a;
     const float v[kOut] = {f.phi, f.dx, f.dy, f.dz, f.dt};
     for (int o = 0; o < kOut; ++o) t[kOut * b + o] = norm ? (v[o] - S.mean[o]) / S.stdv[o] : v[o];

@@ -37,7 +37,7 @@ constexpr long long kVelChunk = 1ll << 19;    // particles per pass (payload: pa
 
 __device__ __forceinline__ int rec_level(const DevTree& T, int cell)
 {
-    return __ldg(reinterpret_cast<const int*>(T.stencil + 8 * (size_t)cell) + 27) & 255;
+    return __ldg(reinterpret_cast<const int*>(T.stencil + 8 * (size_t)cell) + 29) & 255;
 }
 __device__ __forceinline__ int rec_parent(const DevTree& T, int cell)
 {
