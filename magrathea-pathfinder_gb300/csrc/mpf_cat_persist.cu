@@ -192,10 +192,10 @@ constexpr unsigned long long kSlotNs = 2ull * 1000000000ull;
 template <int ORDER>
 __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanDev D, PropParams P, CatConst K)
 {
-    __shared__ double slot_d[kSlotDoubles * kFastThreads];
-    __shared__ float slot_f[kSlotFloats * kFastThreads];
-    const RaySlots J{slot_d + threadIdx.x, slot_f + threadIdx.x};
+    extern __shared__ double slots[];
+    const RaySlots J(slots, kSlotBytes);
     const int lane = threadIdx.x & 31;
+    const RayLanes R(1, lane);
     const PropOut O{D.steps, nullptr, D.rec, D.status, nullptr};
     unsigned long long* const ctl = D.ctl;
     const unsigned long long cap = (unsigned long long)D.cap;
@@ -262,7 +262,7 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
             // Jacobian; from round 2 on, and for the re-trace, with it
             PropParams Pl = P;
             Pl.jacobian = (retrace || it >= 2) ? 1 : 0;
-            propagate_fast<ORDER, true, false>(T, C, Pl, L, s, O, J);
+            propagate_fast<ORDER, true, false>(T, C, Pl, L, s, O, J, R);
             const double* o = D.rec + (long long)kSourceFields * s;
             if (retrace) {
                 cat_final_jacobian(D.call->rows + (long long)kCatalogueFields * s, o, D.steps[s], D.psteps, 0);
@@ -385,8 +385,10 @@ cudaError_t plan_build(CatPlan& pl, const DevTree& T, const DevCosmo& C, PropPar
     P.ray_stop = D.radius;
     // persistent grid: every SM's resident blocks of the propagate launch bounds
     int bps = 0, sms = 0;
-    e = (pl.order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<1>, kFastThreads, 0)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<2>, kFastThreads, 0);
+    e = (pl.order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<1>, kFastThreads,
+                                                                          kFastThreads * kSlotBytes)
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<2>, kFastThreads,
+                                                                          kFastThreads * kSlotBytes);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl.device);
     if (e != cudaSuccess) return e;
     pl.tpb = kFastThreads;
@@ -437,7 +439,7 @@ cudaError_t plan_build(CatPlan& pl, const DevTree& T, const DevCosmo& C, PropPar
         kp.func = (pl.order == 1) ? (void*)k_cat_persistent<1> : (void*)k_cat_persistent<2>;
         kp.gridDim = dim3((unsigned)pl.grid);
         kp.blockDim = dim3((unsigned)pl.tpb);
-        kp.sharedMemBytes = 0;
+        kp.sharedMemBytes = (unsigned)(pl.tpb * kSlotBytes);
         kp.kernelParams = args;
         kp.extra = nullptr;
         e = cudaGraphAddKernelNode(&pl.pnode, g, deps.data(), deps.size(), &kp);
@@ -472,8 +474,8 @@ std::map<std::tuple<int, const void*, int>, CatTune> g_cat_tune;
 int cat_blocks_per_sm(int order, int tpb)
 {
     int b = 0;
-    const cudaError_t e = (order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<1>, tpb, 0)
-                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<2>, tpb, 0);
+    const cudaError_t e = (order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<1>, tpb, (size_t)tpb * kSlotBytes)
+                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<2>, tpb, (size_t)tpb * kSlotBytes);
     return (e == cudaSuccess && b > 0) ? b : 1;
 }
 
@@ -590,6 +592,7 @@ cudaError_t catalogue_newton_persistent(const DevTree& T, const DevCosmo& Cs, co
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     kp.blockDim = dim3((unsigned)tpb);
+    kp.sharedMemBytes = (unsigned)(tpb * kSlotBytes);
     kp.gridDim = dim3((unsigned)(cat_blocks_per_sm(order, tpb) * sms));
     e = cudaGraphExecKernelNodeSetParams(pl.exec, pl.pnode, &kp);
     if (e != cudaSuccess) return e;

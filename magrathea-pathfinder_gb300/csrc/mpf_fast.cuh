@@ -816,34 +816,94 @@ __device__ __forceinline__ Field7 gather_spot(const DevTree& T, const Spot& d, c
     return r;
 }
 
+// Per-thread values that a step touches once, kept in shared memory so that
+// they do not occupy registers through the gathers; one block of slots per
+// warp (dynamic shared memory, kSlotBytes a thread).  S: the Jacobian's FP64 running sums; ck, ckm1: the last point's
+// contribution to them and the one before it (FP32 products of the point's
+// FP32 Hessian terms); cen: the centre of the point's cell; the running
+// integrals of the ray; the comoving distances of the last two points before
+// the current one; the last step's length and change of phi.
+constexpr int kSlotDoubles = 16;
+constexpr int kSlotFloats = 14;
+constexpr int kSlotBytes = kSlotDoubles * 8 + kSlotFloats * 4;
+// with several lanes a ray, also the field gradients of the six Jacobian points
+constexpr int kSharedRaySlotBytes = kSlotBytes + 18 * 4;
+struct RaySlots {
+    double* d;
+    float* f;
+    __device__ __forceinline__ RaySlots(double* shared, int slot_bytes)
+    {
+        double* const warp = shared + (threadIdx.x >> 5) * (32 * slot_bytes / 8);
+        d = warp + (threadIdx.x & 31);
+        f = reinterpret_cast<float*>(warp + 32 * kSlotDoubles) + (threadIdx.x & 31);
+    }
+    // value q of the ray's Jacobian points: one copy for the ray's lanes
+    __device__ __forceinline__ float& point(int sub, int q) const { return f[(kSlotFloats + q) * 32 - sub]; }
+    __device__ __forceinline__ double& S(int q) const { return d[q * 32]; }
+    __device__ __forceinline__ double& cen(int q) const { return d[(6 + q) * 32]; }
+    __device__ __forceinline__ double& lambda() const { return d[9 * 32]; }
+    __device__ __forceinline__ double& s() const { return d[10 * 32]; }
+    __device__ __forceinline__ double& isw() const { return d[11 * 32]; }
+    __device__ __forceinline__ double& iswold() const { return d[12 * 32]; }
+    __device__ __forceinline__ double& chim1() const { return d[13 * 32]; }
+    __device__ __forceinline__ double& chim2() const { return d[14 * 32]; }
+    __device__ __forceinline__ double& last_dl() const { return d[15 * 32]; }
+    __device__ __forceinline__ float& ck(int q) const { return f[q * 32]; }
+    __device__ __forceinline__ float& ckm1(int q) const { return f[(6 + q) * 32]; }
+    __device__ __forceinline__ float& last_dphi() const { return f[12 * 32]; }
+    __device__ __forceinline__ float& rmax() const { return f[13 * 32]; }
+};
+
+// The lanes that trace one ray: a full warp has one ray a lane; a warp with
+// few rays gives each of them 2, 3 or 6 lanes, which take the same steps with
+// the same values (and write the same outputs) and share out the six gathers
+// of the Jacobian, the larger part of a step.
+struct RayLanes {
+    int per_ray;     // 1, 2, 3 or 6
+    int sub;         // this lane's place among them
+    unsigned mask;   // the lanes of the ray
+    __device__ __forceinline__ RayLanes(int lanes_per_ray, int lane)
+        : per_ray(lanes_per_ray), sub(lane % lanes_per_ray), mask(((1u << lanes_per_ray) - 1u) << (lane - lane % lanes_per_ray)) {}
+};
+
 // Jacobian terms (d1d1, d1d2, d2d2 of lensing.h:430-447) at a trajectory
 // point located at `here`: six TSC gathers at +-1 cell of the point's level,
-// the same in-cell offset in the neighbouring cell of the record.
-__device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, double x, double y, double z, float* out3)
+// the same in-cell offset in the neighbouring cell of the record.  With
+// several lanes tracing the ray together each gathers its share of the six.
+__device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, double x, double y, double z, float* out3,
+                                         const RaySlots& J, const RayLanes& R)
 {
     // differences of the plus and minus points, before 1 / dl
     float dxx = 0.f, dxy = 0.f, dxz = 0.f, dyy = 0.f, dyz = 0.f, dzz = 0.f;
+    float mx = 0.f, my = 0.f, mz = 0.f;
 #pragma unroll 1
-    for (int axis = 0; axis < 3; ++axis) {
-        float mx = 0.f, my = 0.f, mz = 0.f;
-#pragma unroll 1
-        for (int sgn = -1; sgn <= 1; sgn += 2) {
-            const int ox = axis == 0 ? sgn : 0, oy = axis == 1 ? sgn : 0, oz = axis == 2 ? sgn : 0;
-            const PosShift pos{x, y, z, here.level, axis, sgn};
-            Spot d;
-            int4 r7;
-            find_spot(T, here, ox, oy, oz, here.f[0], here.f[1], here.f[2], pos, d, r7);
-            const Field7 f = gather_spot<2, false>(T, d, r7, pos, false, nullptr);
-            if (sgn < 0) {
-                mx = f.dx; my = f.dy; mz = f.dz;
-            } else if (axis == 0) {
-                dxx = f.dx - mx;
-            } else if (axis == 1) {
-                dxy = f.dx - mx; dyy = f.dy - my;
-            } else {
-                dxz = f.dx - mx; dyz = f.dy - my; dzz = f.dz - mz;
-            }
+    for (int q = R.sub; q < 6; q += R.per_ray) {
+        const int axis = q >> 1, sgn = (q & 1) ? 1 : -1;
+        const int ox = axis == 0 ? sgn : 0, oy = axis == 1 ? sgn : 0, oz = axis == 2 ? sgn : 0;
+        const PosShift pos{x, y, z, here.level, axis, sgn};
+        Spot d;
+        int4 r7;
+        find_spot(T, here, ox, oy, oz, here.f[0], here.f[1], here.f[2], pos, d, r7);
+        const Field7 f = gather_spot<2, false>(T, d, r7, pos, false, nullptr);
+        if (R.per_ray > 1) {
+            J.point(R.sub, 3 * q) = f.dx; J.point(R.sub, 3 * q + 1) = f.dy; J.point(R.sub, 3 * q + 2) = f.dz;
+        } else if (sgn < 0) {
+            mx = f.dx; my = f.dy; mz = f.dz;
+        } else if (axis == 0) {
+            dxx = f.dx - mx;
+        } else if (axis == 1) {
+            dxy = f.dx - mx; dyy = f.dy - my;
+        } else {
+            dxz = f.dx - mx; dyz = f.dy - my; dzz = f.dz - mz;
         }
+    }
+    if (R.per_ray > 1) {
+        __syncwarp(R.mask);
+        dxx = J.point(R.sub, 3) - J.point(R.sub, 0);
+        dxy = J.point(R.sub, 9) - J.point(R.sub, 6); dyy = J.point(R.sub, 10) - J.point(R.sub, 7);
+        dxz = J.point(R.sub, 15) - J.point(R.sub, 12); dyz = J.point(R.sub, 16) - J.point(R.sub, 13);
+        dzz = J.point(R.sub, 17) - J.point(R.sub, 14);
+        __syncwarp(R.mask);
     }
     // dl = 2^-(level - 1 - log2 EXTENT) (lensing.h:430), twice the shift
     const float idl = __int_as_float((127 + here.level - kLevelShift - 1) << 23);   // 1 / dl, exact
@@ -860,33 +920,6 @@ __device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, dou
               cp * s2t * dxz;
 }
 
-// Per-thread values that a step touches once, kept in shared memory so that
-// they do not occupy registers through the gathers; strided by the block
-// size.  S: the Jacobian's FP64 running sums; ck, ckm1: the last point's
-// contribution to them and the one before it (FP32 products of the point's
-// FP32 Hessian terms); cen: the centre of the point's cell; the running
-// integrals of the ray; the comoving distances of the last two points before
-// the current one; the last step's length and change of phi.
-constexpr int kSlotDoubles = 16;
-constexpr int kSlotFloats = 14;
-struct RaySlots {
-    double* d;
-    float* f;
-    __device__ __forceinline__ double& S(int q) const { return d[q * kFastThreads]; }
-    __device__ __forceinline__ double& cen(int q) const { return d[(6 + q) * kFastThreads]; }
-    __device__ __forceinline__ double& lambda() const { return d[9 * kFastThreads]; }
-    __device__ __forceinline__ double& s() const { return d[10 * kFastThreads]; }
-    __device__ __forceinline__ double& isw() const { return d[11 * kFastThreads]; }
-    __device__ __forceinline__ double& iswold() const { return d[12 * kFastThreads]; }
-    __device__ __forceinline__ double& chim1() const { return d[13 * kFastThreads]; }
-    __device__ __forceinline__ double& chim2() const { return d[14 * kFastThreads]; }
-    __device__ __forceinline__ double& last_dl() const { return d[15 * kFastThreads]; }
-    __device__ __forceinline__ float& ck(int q) const { return f[q * kFastThreads]; }
-    __device__ __forceinline__ float& ckm1(int q) const { return f[(6 + q) * kFastThreads]; }
-    __device__ __forceinline__ float& last_dphi() const { return f[12 * kFastThreads]; }
-    __device__ __forceinline__ float& rmax() const { return f[13 * kFastThreads]; }
-};
-
 // a trajectory point's state and the field there
 struct RayPoint {
     double a, t, x, y, z, k0, k1, k2, k3, chi;
@@ -902,7 +935,7 @@ struct RayPoint {
 // (integrator.h:707-708, 765-767); plain instantiations only.
 template <int ORDER, bool SRC, bool WIDE, bool BORN = false, bool VEL = false>
 __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropParams& P, const double* L, long long i,
-                               const PropOut& O, RaySlots J)
+                               const PropOut& O, const RaySlots& J, const RayLanes& R)
 {
     const double c2 = kC * kC;
     const double mn = -(double)kExtent / 2.0, mx = (double)kExtent / 2.0;
@@ -1287,7 +1320,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         here = q;
         if (P.jacobian) {
             float h3[3];
-            jac_fast(T, here, b.x, b.y, b.z, h3);
+            jac_fast(T, here, b.x, b.y, b.z, h3, J, R);
             const float chif = (float)b.chi;
             J.chim2() = J.chim1();
             J.chim1() = chi_b;
@@ -1412,11 +1445,12 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     if (status) atomicOr(O.status, status);
 }
 
-// Persistent launch: each warp takes the next 32 x depth rays of [lo, n) from
-// a global counter until the range is exhausted, so uneven path lengths do
-// not leave tail waves; its lanes trace them depth at a time.  `queue` is
-// zeroed before the launch.  The block size and depth are the autotuner's
-// (mpf_prop_fast.cu); the rays' results do not depend on them.
+// Persistent launch: each warp takes the next rays x depth rays of [lo, n)
+// from a global counter until the range is exhausted, so uneven path lengths
+// do not leave tail waves; it traces `rays` of them at a time with per_ray
+// lanes each (rays x per_ray <= 32).  `queue` is zeroed before the launch.
+// The launch shape is the launcher's (mpf_prop_fast.cu); the rays' results do
+// not depend on it.
 #if defined(MPF_FAST_MAXNREG)
 #define MPF_FAST_BOUNDS __maxnreg__(MPF_FAST_MAXNREG)
 #else
@@ -1425,21 +1459,23 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
 template <int ORDER, bool SRC, bool WIDE, bool BORN = false, bool VEL = false>
 __global__ void MPF_FAST_BOUNDS k_propagate_fast(DevTree T, DevCosmo C, PropParams P,
                                                                     const double* __restrict__ launch, long long n, PropOut O,
-                                                                    unsigned long long* queue, int depth, long long lo)
+                                                                    unsigned long long* queue, int rays, int per_ray, int depth,
+                                                                    long long lo)
 {
-    __shared__ double slot_d[kSlotDoubles * kFastThreads];
-    __shared__ float slot_f[kSlotFloats * kFastThreads];
-    const RaySlots J{slot_d + threadIdx.x, slot_f + threadIdx.x};
+    extern __shared__ double slots[];
+    const RaySlots J(slots, per_ray > 1 ? kSharedRaySlotBytes : kSlotBytes);
     const int lane = threadIdx.x & 31;
-    const unsigned long long per = 32ull * (unsigned long long)depth;
+    const RayLanes R(per_ray, lane);
+    const int ray = lane / per_ray;
+    const unsigned long long per = (unsigned long long)rays * (unsigned long long)depth;
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(queue, per);
         base = __shfl_sync(0xffffffffu, base, 0) + (unsigned long long)lo;
         if (base >= (unsigned long long)n) break;
         for (int d = 0; d < depth; ++d) {
-            const long long i = (long long)base + 32ll * d + lane;
-            if (i < n) propagate_fast<ORDER, SRC, WIDE, BORN, VEL>(T, C, P, launch + 6 * i, i, O, J);
+            const long long i = (long long)base + (long long)rays * d + ray;
+            if (ray < rays && i < n) propagate_fast<ORDER, SRC, WIDE, BORN, VEL>(T, C, P, launch + 6 * i, i, O, J, R);
             __syncwarp();
         }
     }

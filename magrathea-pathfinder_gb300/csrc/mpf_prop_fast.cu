@@ -37,47 +37,53 @@ static bool fast_mode_supported(const DevTree& T, const PropParams& P, const Pro
 }
 
 // Launches rays [lo, n) of the batch as grid blocks of tpb threads, each warp
-// claiming 32 x depth rays at a time.
-static void launch_fast_kernel(long long grid, int tpb, int depth, long long lo, const DevTree& T, const DevCosmo& C,
+// claiming rays x depth rays at a time and tracing them with per_ray lanes each.
+static void launch_fast_kernel(long long grid, int tpb, int rays, int per_ray, int depth, long long lo, const DevTree& T, const DevCosmo& C,
                                const PropParams& P, const double* d_launch, long long n, const PropOut& O,
                                unsigned long long* queue, cudaStream_t stream)
 {
     const unsigned g = (unsigned)grid;
+    const size_t smem = (size_t)tpb * (per_ray > 1 ? kSharedRaySlotBytes : kSlotBytes);
     switch (fast_mode(T, P, O)) {
     // Born rays: the field is homogeneous, so the interpolation order does
     // not enter (the Jacobian gathers are TSC)
-    case 0: k_propagate_fast<2, true, false, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 1: k_propagate_fast<2, false, true, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 2: k_propagate_fast<1, true, false><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 3: k_propagate_fast<2, true, false><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 4: k_propagate_fast<1, false, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 5: k_propagate_fast<2, false, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 6: k_propagate_fast<1, false, false><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 8: k_propagate_fast<1, false, false, false, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    case 9: k_propagate_fast<2, false, false, false, true><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
-    default: k_propagate_fast<2, false, false><<<g, tpb, 0, stream>>>(T, C, P, d_launch, n, O, queue, depth, lo); break;
+    case 0: k_propagate_fast<2, true, false, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 1: k_propagate_fast<2, false, true, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 2: k_propagate_fast<1, true, false><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 3: k_propagate_fast<2, true, false><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 4: k_propagate_fast<1, false, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 5: k_propagate_fast<2, false, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 6: k_propagate_fast<1, false, false><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 8: k_propagate_fast<1, false, false, false, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    case 9: k_propagate_fast<2, false, false, false, true><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
+    default: k_propagate_fast<2, false, false><<<g, tpb, smem, stream>>>(T, C, P, d_launch, n, O, queue, rays, per_ray, depth, lo); break;
     }
 }
 
-// Launch shape of the persistent kernel.  A batch that fills every SM's
-// warp slots runs as blocks of kFastThreads, as many as are resident.  A
-// smaller one (the catalogue's last Newton rounds, small ray batches) runs as
-// one-warp blocks, one per 32 rays, so that the block scheduler spreads its
-// warps over the SMs instead of packing four to an SM: each warp then has an
-// SM's FP64 pipe and load slots to itself and its rays finish sooner.
-// The kernel's shared-memory layout is sized for kFastThreads and takes any
-// smaller block.
-static int fast_launch_shape(long long n, int blocks_per_sm, int sms, long long* grid)
+// Launch shape of the persistent kernel.  A ray's steps are one serial chain,
+// and what a warp spends on a step grows with the rays in it (other cells,
+// levels, table intervals and step counts: 32.6 ms for one ray a warp, 46 for
+// 16, 60 to 72 for 32 on a refined cone with the Jacobian) and with the warps
+// that share its SM sub-partition.  So a batch of fewer rays than one full
+// warp per sub-partition is spread over one-warp blocks, one per
+// sub-partition (4 an SM; two a sub-partition measured 48 -> 79 ms at 4096
+// rays, half a warp each 48 -> 55), with the rays' Jacobian gathers shared out
+// to the lanes left over.  Above that, blocks of one warp while they do not
+// fill the warp slots, then blocks of kFastThreads, as many as are resident.
+struct FastShape {
+    long long grid;
+    int tpb;
+    int rays, per_ray;   // rays of a warp, lanes of a ray
+    bool full;           // blocks of kFastThreads: the autotuner's case
+};
+static FastShape fast_launch_shape(long long n, int blocks_per_sm, int sms, bool jacobian)
 {
-    const long long warps = (n + 31) / 32;
     const long long slots = (long long)blocks_per_sm * sms * (kFastThreads / 32);
-    if (warps < slots) {
-        *grid = warps;
-        return 32;
-    }
-    const long long need = (n + kFastThreads - 1) / kFastThreads;
-    *grid = std::min<long long>(need, (long long)blocks_per_sm * sms);
-    return kFastThreads;
+    const int rays = (int)std::min<long long>(32, (n + 4 * sms - 1) / (4 * sms));
+    const int per_ray = !jacobian ? 1 : (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1;
+    const long long warps = (n + rays - 1) / rays;
+    if (warps < slots) return FastShape{warps, 32, rays, per_ray, false};
+    return FastShape{std::min<long long>((n + kFastThreads - 1) / kFastThreads, (long long)blocks_per_sm * sms), kFastThreads, 32, 1, true};
 }
 
 // Work-queue counter and occupancy of the persistent kernel, per (device,
@@ -104,7 +110,7 @@ static cudaError_t fast_launch_state(cudaStream_t stream, FastLaunchState* out)
     std::lock_guard<std::mutex> lock(mu);
     FastLaunchState& s = states[std::make_tuple(dev, stream, who)];
     if (!s.queue) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.blocks_per_sm, k_propagate_fast<2, false, false>, kFastThreads, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.blocks_per_sm, k_propagate_fast<2, false, false>, kFastThreads, kFastThreads * kSlotBytes);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess) e = cudaMalloc(&s.queue, sizeof(unsigned long long));
         if (e != cudaSuccess) {
@@ -156,7 +162,7 @@ static __global__ void k_sum_steps(const long long* __restrict__ steps, long lon
 static int blocks_per_sm_at(int tpb)
 {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_propagate_fast<2, false, false>, tpb, 0) != cudaSuccess) b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_propagate_fast<2, false, false>, tpb, (size_t)tpb * kSlotBytes) != cudaSuccess) b = 1;
     return std::max(1, b);
 }
 
@@ -185,7 +191,7 @@ static cudaError_t tune_and_launch(const DevTree& T, const DevCosmo& C, const Pr
         const TuneShape& sh = kTuneCandidates[k];
         e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), stream);
         if (e != cudaSuccess) break;
-        launch_fast_kernel(shape_grid(sh, hi - lo, sms), sh.tpb, sh.depth, lo, T, C, P, d_launch, hi, O, queue, stream);
+        launch_fast_kernel(shape_grid(sh, hi - lo, sms), sh.tpb, 32, 1, sh.depth, lo, T, C, P, d_launch, hi, O, queue, stream);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         e = cudaEventRecord(ev[k + 1], stream);
         if (e == cudaSuccess) k_sum_steps<<<64, 256, 0, stream>>>(O.steps, lo, hi, dsum + k);
@@ -254,15 +260,14 @@ cudaError_t launch_propagate<false>(const DevTree& T, const DevCosmo& C, const P
     unsigned long long* const queue = st.queue;
     e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
-    long long grid = 0;
-    int tpb_used = fast_launch_shape(n, st.blocks_per_sm, st.sms, &grid);
+    FastShape shape = fast_launch_shape(n, st.blocks_per_sm, st.sms, P.jacobian != 0);
     int depth = 1;
 #if MPF_DIAG
     // MPF_STATS=1: print the counts of the rare paths (diagnostics; serialises the call)
     static const bool want_stats = getenv("MPF_STATS") != nullptr;
 #endif
     static const bool want_tune = !(getenv("MPF_AUTOTUNE") && getenv("MPF_AUTOTUNE")[0] == '0');
-    if (tpb_used == kFastThreads && want_tune) {
+    if (shape.full && want_tune) {
         // a batch that fills the GPU: the tuned shape of this octree and kernel mode
         int dev = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -286,12 +291,12 @@ cudaError_t launch_propagate<false>(const DevTree& T, const DevCosmo& C, const P
             return e;
         }
         if (have) {
-            tpb_used = res.best.tpb;
+            shape.tpb = res.best.tpb;
             depth = res.best.depth;
-            grid = shape_grid(res.best, n, st.sms);
+            shape.grid = shape_grid(res.best, n, st.sms);
         }
     }
-    launch_fast_kernel(grid, tpb_used, depth, 0, T, C, P, d_launch, n, O, queue, stream);
+    launch_fast_kernel(shape.grid, shape.tpb, shape.rays, shape.per_ray, depth, 0, T, C, P, d_launch, n, O, queue, stream);
     e = cudaGetLastError();
 #if MPF_DIAG
     if (want_stats) {
@@ -321,14 +326,13 @@ cudaError_t launch_propagate_fast_with_queue(const DevTree& T, const DevCosmo& C
     if (n <= 0) return cudaSuccess;
     const int tpb = kFastThreads;
     int blocks_per_sm = 0, sms = 0, dev = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_propagate_fast<2, false, false>, tpb, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_propagate_fast<2, false, false>, tpb, (size_t)tpb * kSlotBytes);
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     if (blocks_per_sm < 1) blocks_per_sm = 1;
-    long long grid = 0;
-    const int tpb_used = fast_launch_shape(n, blocks_per_sm, sms, &grid);
-    launch_fast_kernel(grid, tpb_used, 1, 0, T, C, P, d_launch, n, O, queue, stream);
+    const FastShape shape = fast_launch_shape(n, blocks_per_sm, sms, P.jacobian != 0);
+    launch_fast_kernel(shape.grid, shape.tpb, shape.rays, shape.per_ray, 1, 0, T, C, P, d_launch, n, O, queue, stream);
     return cudaGetLastError();
 }
 }  // namespace mpf
