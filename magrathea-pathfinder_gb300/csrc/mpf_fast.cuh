@@ -128,17 +128,17 @@ __device__ unsigned long long g_diag[4];
 // so that the hot loop stays small in the instruction cache.
 static __device__ __noinline__ Field7 tsc_slow(const DevTree& T, double x, double y, double z, int need_all)
 {
-    return tsc<false>(T, x, y, z, need_all != 0);
+    return tsc(T, x, y, z, need_all != 0);
 }
 static __device__ __noinline__ Field7 cic_slow(const DevTree& T, double x, double y, double z, int need_all)
 {
-    return cic<false>(T, x, y, z, need_all != 0);
+    return cic(T, x, y, z, need_all != 0);
 }
 static __device__ __noinline__ Found locate_slow(const DevTree& T, double x, double y, double z) { return locate(T, x, y, z); }
 // the 7 fields and the velocity, full walk (velocity-field octrees)
 static __device__ __noinline__ Field7 vel_slow(const DevTree& T, int order, double x, double y, double z, float* v)
 {
-    return gather_vel<false>(T, order, x, y, z, v);
+    return gather_vel(T, order, x, y, z, v);
 }
 
 // A point given by its float64 coordinates.

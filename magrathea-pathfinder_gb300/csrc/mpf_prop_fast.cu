@@ -1,7 +1,7 @@
 // Throughput mode: FP32 gather arithmetic through the per-cell stencil
 // records, FP64 RK4 state (with FMA).
 #include "mpf_fast.cuh"
-#include "mpf_prop_impl.cuh"
+#include "mpf_internal.h"
 
 #include <algorithm>
 #include <cstdio>

@@ -1,4 +1,4 @@
-"""Launch shapes of the FP32-gather kernel: a batch smaller than one full warp
+"""Launch shapes of the propagation kernels: a batch smaller than one full warp
 per SM sub-partition runs with fewer rays a warp and, with the Jacobian, with
 2, 3 or 6 lanes a ray.  A ray's result does not depend on the shape, so the
 first n rays traced alone equal bit for bit the same rays of a batch that
@@ -33,6 +33,21 @@ def test_small_batches_equal_large_ones(rays, pkg, order, jacobian, n):
     if (order, jacobian) not in whole:
         whole[order, jacobian] = pkg.propagate(tree, cos, launch, length, **kw)
     s0, f0, p0, _ = whole[order, jacobian]
+    s, f, p, rc = pkg.propagate(tree, cos, launch[:n], length, **kw)
+    assert rc == 0
+    np.testing.assert_array_equal(s, s0[:n])
+    np.testing.assert_array_equal(f.view(np.uint64), f0[:n].view(np.uint64))
+    np.testing.assert_array_equal(p.view(np.uint64), p0[:n].view(np.uint64))
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("n", (1, 609, 3041, 6081, 9729))
+def test_small_exact_batches_equal_large_ones(rays, pkg, order, n):
+    tree, cos, length, launch, whole = rays
+    kw = dict(nsteps=4, order=order, stop="redshift", stop_value=0.03, planes=np.array([0.01, 0.03]), jacobian=True, exact=True)
+    if ("exact", order) not in whole:
+        whole["exact", order] = pkg.propagate(tree, cos, launch, length, **kw)
+    s0, f0, p0, _ = whole["exact", order]
     s, f, p, rc = pkg.propagate(tree, cos, launch[:n], length, **kw)
     assert rc == 0
     np.testing.assert_array_equal(s, s0[:n])
