@@ -249,6 +249,9 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
                 __nanosleep(64);
             }
         }
+        // the item's state was written by the warp that queued it, on any SM:
+        // nothing of it may come from this SM's L1
+        __threadfence();
         int push = -1;
         if (item >= 0) {
             const int s = item >> 1;
@@ -277,6 +280,9 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
                 }
             }
         }
+        // the sources' states and records are visible to the warps that take
+        // them from the queue
+        __threadfence();
         // warp-aggregated push of the sources that need another ray
         const unsigned want = __ballot_sync(0xffffffffu, push >= 0);
         if (want) {
