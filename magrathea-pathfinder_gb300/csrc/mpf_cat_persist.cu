@@ -193,9 +193,9 @@ template <int ORDER>
 __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanDev D, PropParams P, CatConst K)
 {
     extern __shared__ double slots[];
-    const RaySlots J(slots, kSlotBytes);
+    const RaySlots J(slots, kSharedRaySlotBytes);
     const int lane = threadIdx.x & 31;
-    const RayLanes R(1, lane);
+    const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     const PropOut O{D.steps, nullptr, D.rec, D.status, nullptr};
     unsigned long long* const ctl = D.ctl;
     const unsigned long long cap = (unsigned long long)D.cap;
@@ -210,7 +210,11 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
                 const unsigned long long h = atomicAdd(ctl + kQHead, 0ull);
                 const unsigned long long t = atomicAdd(ctl + kQTail, 0ull);
                 if (h < t) {
-                    const unsigned long long c = min(32ull, t - h);
+                    // no more than this warp's share of the sources still at
+                    // work: fewer rays a warp finish sooner (500 sources 216 ->
+                    // 120 ms, 16384 293 -> 205, 70 000 345 -> 288 a call against
+                    // 32 rays a warp throughout)
+                    const unsigned long long c = min(min(32ull, (t - h + fl + warps - 1) / warps), t - h);
                     atomicAdd(ctl + kQFlight, c);
                     if (atomicCAS(ctl + kQHead, h, h + c) == h) {
                         base = h;
@@ -228,9 +232,13 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
         base = __shfl_sync(0xffffffffu, base, 0);
         cnt = __shfl_sync(0xffffffffu, cnt, 0);
         if (cnt == 0) break;
+        // a warp with few rays traces each with several lanes (RayLanes); the
+        // first of them takes the item and makes the Newton update
+        const RayLanes R(rays_to_lanes(cnt), lane);
+        const int ray = lane / R.per_ray;
         int item = -1;
-        if (lane < cnt) {
-            const unsigned long long pos = base + (unsigned long long)lane;
+        if (ray < cnt && R.sub == 0) {
+            const unsigned long long pos = base + (unsigned long long)ray;
             const unsigned long long lap = pos / cap;
             unsigned long long* const sw = D.items + (long long)(pos % cap);
             const unsigned long long t0 = global_ns();
@@ -252,6 +260,8 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
         // the item's state was written by the warp that queued it, on any SM:
         // nothing of it may come from this SM's L1
         __threadfence();
+        item = __shfl_sync(0xffffffffu, item, lane - R.sub);
+        if (ray >= cnt) item = -1;
         int push = -1;
         if (item >= 0) {
             const int s = item >> 1;
@@ -266,8 +276,11 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
             PropParams Pl = P;
             Pl.jacobian = (retrace || it >= 2) ? 1 : 0;
             propagate_fast<ORDER, true, false>(T, C, Pl, L, s, O, J, R);
+            __syncwarp(R.mask);   // every lane has read the state
             const double* o = D.rec + (long long)kSourceFields * s;
-            if (retrace) {
+            if (R.sub != 0) {
+                // the ray's first lane goes on alone
+            } else if (retrace) {
                 cat_final_jacobian(D.call->rows + (long long)kCatalogueFields * s, o, D.steps[s], D.psteps, 0);
             } else {
                 const int r = cat_update(s, it, Pl.jacobian, K, D.state, D.call->rows, D.steps[s], o, D.psteps);
@@ -313,7 +326,7 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
                 }
             }
         }
-        const unsigned traced = __ballot_sync(0xffffffffu, item >= 0);
+        const unsigned traced = __ballot_sync(0xffffffffu, item >= 0 && R.sub == 0);
         __threadfence();
         __syncwarp();
         if (lane == 0) {
@@ -392,9 +405,9 @@ cudaError_t plan_build(CatPlan& pl, const DevTree& T, const DevCosmo& C, PropPar
     // persistent grid: every SM's resident blocks of the propagate launch bounds
     int bps = 0, sms = 0;
     e = (pl.order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<1>, kFastThreads,
-                                                                          kFastThreads * kSlotBytes)
+                                                                          kFastThreads * kSharedRaySlotBytes)
                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<2>, kFastThreads,
-                                                                          kFastThreads * kSlotBytes);
+                                                                          kFastThreads * kSharedRaySlotBytes);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl.device);
     if (e != cudaSuccess) return e;
     pl.tpb = kFastThreads;
@@ -445,7 +458,7 @@ cudaError_t plan_build(CatPlan& pl, const DevTree& T, const DevCosmo& C, PropPar
         kp.func = (pl.order == 1) ? (void*)k_cat_persistent<1> : (void*)k_cat_persistent<2>;
         kp.gridDim = dim3((unsigned)pl.grid);
         kp.blockDim = dim3((unsigned)pl.tpb);
-        kp.sharedMemBytes = (unsigned)(pl.tpb * kSlotBytes);
+        kp.sharedMemBytes = (unsigned)(pl.tpb * kSharedRaySlotBytes);
         kp.kernelParams = args;
         kp.extra = nullptr;
         e = cudaGraphAddKernelNode(&pl.pnode, g, deps.data(), deps.size(), &kp);
@@ -480,8 +493,8 @@ std::map<std::tuple<int, const void*, int>, CatTune> g_cat_tune;
 int cat_blocks_per_sm(int order, int tpb)
 {
     int b = 0;
-    const cudaError_t e = (order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<1>, tpb, (size_t)tpb * kSlotBytes)
-                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<2>, tpb, (size_t)tpb * kSlotBytes);
+    const cudaError_t e = (order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<1>, tpb, (size_t)tpb * kSharedRaySlotBytes)
+                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cat_persistent<2>, tpb, (size_t)tpb * kSharedRaySlotBytes);
     return (e == cudaSuccess && b > 0) ? b : 1;
 }
 
@@ -598,8 +611,15 @@ cudaError_t catalogue_newton_persistent(const DevTree& T, const DevCosmo& Cs, co
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     kp.blockDim = dim3((unsigned)tpb);
-    kp.sharedMemBytes = (unsigned)(tpb * kSlotBytes);
+    kp.sharedMemBytes = (unsigned)(tpb * kSharedRaySlotBytes);
     kp.gridDim = dim3((unsigned)(cat_blocks_per_sm(order, tpb) * sms));
+    if (n <= 128ll * sms) {
+        // fewer sources than a full warp per SM sub-partition: one warp on each
+        // (the launch rule of the propagation kernel)
+        kp.blockDim = dim3(32u);
+        kp.sharedMemBytes = (unsigned)(32 * kSharedRaySlotBytes);
+        kp.gridDim = dim3((unsigned)(4 * sms));
+    }
     e = cudaGraphExecKernelNodeSetParams(pl.exec, pl.pnode, &kp);
     if (e != cudaSuccess) return e;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -858,6 +858,7 @@ struct RaySlots {
 // few rays gives each of them 2, 3 or 6 lanes, which take the same steps with
 // the same values (and write the same outputs) and share out the six gathers
 // of the Jacobian, the larger part of a step.
+__host__ __device__ __forceinline__ int rays_to_lanes(int rays) { return (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1; }
 struct RayLanes {
     int per_ray;     // 1, 2, 3 or 6
     int sub;         // this lane's place among them

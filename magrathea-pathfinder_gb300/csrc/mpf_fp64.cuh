@@ -1,0 +1,67 @@
+// float64 operations on the integer bits.  An SM sub-partition's FP64 pipe
+// takes a warp's add, multiply, fused multiply-add, compare or conversion 64
+// cycles, however many of its lanes are active (measured; the integer and FP32
+// pipes take 1 to 2); the functions below give the bits of the hardware's
+// conversions, products with powers of two and compares in 4 to 10 integer
+// instructions, and leave zeros, subnormals, infinities and NaN to it.
+#pragma once
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace mpf {
+
+// (double)v
+__device__ __forceinline__ double wide(float v)
+{
+    const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
+    if (a - 0x00800000u < 0x7f000000u)
+        return __hiloint2double((int)(((a >> 3) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
+    return (double)v;
+}
+
+// Range of the high word's magnitude whose value rounds to a normal float
+// below 2^127: exponents -126 to 126.
+__device__ __forceinline__ bool normal_float_range(unsigned hi) { return (hi & 0x7fffffffu) - 0x38100000u < 0x47e00000u - 0x38100000u; }
+
+// (float)d: round to nearest even at bit 29
+__device__ __forceinline__ float narrow(double d)
+{
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    if (normal_float_range(hi)) {
+        const unsigned l2 = lo + 0x0fffffffu + ((lo >> 29) & 1u);
+        const unsigned h2 = (hi & 0x7fffffffu) - 0x38000000u + (l2 < lo ? 1u : 0u);
+        return __uint_as_float(__funnelshift_l(l2, h2, 3) | (hi & 0x80000000u));
+    }
+    return __double2float_rn(d);
+}
+
+// (double)(float)d
+__device__ __forceinline__ double round32(double d)
+{
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    if (normal_float_range(hi)) {
+        const unsigned l2 = lo + 0x0fffffffu + ((lo >> 29) & 1u);
+        return __hiloint2double((int)(hi + (l2 < lo ? 1u : 0u)), (int)(l2 & 0xe0000000u));
+    }
+    return (double)__double2float_rn(d);
+}
+
+// d * 2^e (|e| < 512)
+__device__ __forceinline__ double times_pow2(double d, int e)
+{
+    const unsigned hi = (unsigned)__double2hiint(d);
+    if ((hi & 0x7fffffffu) - 0x20000000u < 0x3fe00000u) return __hiloint2double((int)(hi + ((unsigned)e << 20)), __double2loint(d));
+    return d * __longlong_as_double((long long)(1023 + e) << 52);
+}
+
+// a < b for numbers (of two zeros the negative one is the smaller; a NaN is
+// beyond the infinity of its sign)
+__device__ __forceinline__ bool less64(double a, double b)
+{
+    long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    x ^= (long long)((unsigned long long)(x >> 63) >> 1);
+    y ^= (long long)((unsigned long long)(y >> 63) >> 1);
+    return x < y;
+}
+
+}  // namespace mpf

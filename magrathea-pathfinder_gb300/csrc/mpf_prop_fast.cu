@@ -80,7 +80,7 @@ static FastShape fast_launch_shape(long long n, int blocks_per_sm, int sms, bool
 {
     const long long slots = (long long)blocks_per_sm * sms * (kFastThreads / 32);
     const int rays = (int)std::min<long long>(32, (n + 4 * sms - 1) / (4 * sms));
-    const int per_ray = !jacobian ? 1 : (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1;
+    const int per_ray = jacobian ? rays_to_lanes(rays) : 1;
     const long long warps = (n + rays - 1) / rays;
     if (warps < slots) return FastShape{warps, 32, rays, per_ray, false};
     return FastShape{std::min<long long>((n + kFastThreads - 1) / kFastThreads, (long long)blocks_per_sm * sms), kFastThreads, 32, 1, true};
