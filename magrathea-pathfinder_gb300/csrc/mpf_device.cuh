@@ -49,6 +49,7 @@ struct DevTree {
     const float4* vel;
     int64_t n;
     int Lt;                // level of the top grid
+    int Lmax;              // the finest level
     int gx0, gy0, gz0;     // grid origin (integer coords at Lt)
     int gnx, gny, gnz;     // grid dims
 };

@@ -1450,8 +1450,8 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
 // from a global counter until the range is exhausted, so uneven path lengths
 // do not leave tail waves; it traces `rays` of them at a time with per_ray
 // lanes each (rays x per_ray <= 32).  `queue` is zeroed before the launch.
-// The launch shape is the launcher's (mpf_prop_fast.cu); the rays' results do
-// not depend on it.
+// The launch shape and the order (perm: the ray at each position, or null) are
+// the launcher's (mpf_prop_fast.cu); the rays' results do not depend on them.
 #if defined(MPF_FAST_MAXNREG)
 #define MPF_FAST_BOUNDS __maxnreg__(MPF_FAST_MAXNREG)
 #else
@@ -1461,7 +1461,7 @@ template <int ORDER, bool SRC, bool WIDE, bool BORN = false, bool VEL = false>
 __global__ void MPF_FAST_BOUNDS k_propagate_fast(DevTree T, DevCosmo C, PropParams P,
                                                                     const double* __restrict__ launch, long long n, PropOut O,
                                                                     unsigned long long* queue, int rays, int per_ray, int depth,
-                                                                    long long lo)
+                                                                    long long lo, const int* __restrict__ perm)
 {
     extern __shared__ double slots[];
     const RaySlots J(slots, per_ray > 1 ? kSharedRaySlotBytes : kSlotBytes);
@@ -1475,8 +1475,11 @@ __global__ void MPF_FAST_BOUNDS k_propagate_fast(DevTree T, DevCosmo C, PropPara
         base = __shfl_sync(0xffffffffu, base, 0) + (unsigned long long)lo;
         if (base >= (unsigned long long)n) break;
         for (int d = 0; d < depth; ++d) {
-            const long long i = (long long)base + (long long)rays * d + ray;
-            if (ray < rays && i < n) propagate_fast<ORDER, SRC, WIDE, BORN, VEL>(T, C, P, launch + 6 * i, i, O, J, R);
+            long long i = (long long)base + (long long)rays * d + ray;
+            if (ray < rays && i < n) {
+                if (perm) i = perm[i];
+                propagate_fast<ORDER, SRC, WIDE, BORN, VEL>(T, C, P, launch + 6 * i, i, O, J, R);
+            }
             __syncwarp();
         }
     }

@@ -69,7 +69,7 @@ cudaError_t launch_gather(const DevTree& T, int kind, bool exact, const double* 
 bool tuned_shape(int dev, const DevTree& T, int mode, int* tpb, int* depth, double* rates);
 int plain_fast_mode(int order, bool velocity);
 bool catalogue_tuned_shape(int dev, const DevTree& T, int order, int* tpb, double* rates);
-// forget an octree's tuned shapes when its arrays are freed
+// forget an octree's tuned shapes (and free its ray orders) when its arrays are freed
 void forget_tuned_shape(const void* keys);
 void catalogue_forget_tuned_shape(const void* keys);
 

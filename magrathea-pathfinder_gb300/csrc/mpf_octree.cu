@@ -410,6 +410,7 @@ extern "C" int mpf_internal_octree_build(const void* records, int64_t n, int on_
     o->tree.grid = o->grid;
     o->tree.n = n;
     o->tree.Lt = Lt;
+    o->tree.Lmax = o->level_max;
     o->tree.gx0 = bb[0]; o->tree.gy0 = bb[1]; o->tree.gz0 = bb[2];
     o->tree.gnx = gnx; o->tree.gny = gny; o->tree.gnz = gnz;
     if (!dalloc((void**)&o->stencil, (size_t)n * 8 * sizeof(int4), false)) { release(true); return fail("out of device memory", -2); }

@@ -53,3 +53,23 @@ def test_small_exact_batches_equal_large_ones(rays, pkg, order, n):
     np.testing.assert_array_equal(s, s0[:n])
     np.testing.assert_array_equal(f.view(np.uint64), f0[:n].view(np.uint64))
     np.testing.assert_array_equal(p.view(np.uint64), p0[:n].view(np.uint64))
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("n", (16383, 16384, 40000))
+def test_ray_order_changes_no_ray(rays, pkg, order, n):
+    """From 2^14 rays on a refined octree runs the rays in the order of their
+    directions: any order of the caller's gives the same rays, directions in
+    all eight octants and repeated ones among them."""
+    tree, cos, length, launch, _ = rays
+    rng = np.random.default_rng(n)
+    some = launch[rng.permutation(launch.shape[0])[:n]].copy()
+    some[::1000, 3:] = rng.normal(size=some[::1000, 3:].shape)
+    some[1::1000] = some[0]
+    kw = dict(nsteps=4, order=order, stop="redshift", stop_value=0.04, planes=np.array([0.04]), jacobian=True)
+    s, f, p, _ = pkg.propagate(tree, cos, some, length, **kw)
+    for lo in range(0, n, 8000):     # below the threshold: in the caller's order
+        s0, f0, p0, _ = pkg.propagate(tree, cos, some[lo:lo + 8000], length, **kw)
+        np.testing.assert_array_equal(s[lo:lo + 8000], s0)
+        np.testing.assert_array_equal(f[lo:lo + 8000].view(np.uint64), f0.view(np.uint64))
+        np.testing.assert_array_equal(p[lo:lo + 8000].view(np.uint64), p0.view(np.uint64))
