@@ -305,15 +305,16 @@ def cells_build(rows, cosmology: Cosmology, cone_vertex, cone_base, cone_angle, 
     amin = np.zeros(1)
     p.acorrection, p.order, p.amin = int(bool(acorrection)), int(order), amin.ctypes.data
     cap = 2 * rows.shape[0] + 64
-    out = np.zeros(cap * 48, dtype=np.uint8)
+    out = np.empty(cap * 48, dtype=np.uint8)
     n = C.c_int64()
     rc = L.mpf_cells_build(capi.ptr(rows), rows.shape[0], C.byref(p), cosmology._h, capi.ptr(out), cap, C.byref(n))
     if rc == -1 and n.value > cap:   # MPF_BAD_INPUT: more cells than the first guess; build again at the size
         cap = n.value
-        out = np.zeros(cap * 48, dtype=np.uint8)
+        out = np.empty(cap * 48, dtype=np.uint8)
         rc = L.mpf_cells_build(capi.ptr(rows), rows.shape[0], C.byref(p), cosmology._h, capi.ptr(out), cap, C.byref(n))
     capi.check(rc)
-    rec = out[:48 * n.value].copy()
+    out.resize(48 * n.value, refcheck=False)   # gives the rest back without a copy
+    rec = out
     return (rec, float(amin[0])) if acorrection else rec
 
 

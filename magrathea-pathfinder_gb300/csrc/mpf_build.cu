@@ -36,6 +36,7 @@
 
 #include "../../include/mpf_gb300.h"
 #include "mpf_internal.h"
+#include "mpf_sort.cuh"
 
 namespace mpf {
 namespace build {
@@ -155,50 +156,40 @@ __global__ void k_sistemize(long long n, Rec48* r, Geometry G)
     r[i].dt = 0.f;
 }
 
-// ---- stable LSD radix sort of (hi, lo) with the record index as payload ----
-constexpr int kTile = 256;
-__global__ void k_keys(long long n, const Rec48* __restrict__ r, unsigned long long* hi, unsigned long long* lo, int* idx)
+// ---- stable sort by key with the record index as payload ----
+// one half of the keys, in the payload's order (idx null: the records' own)
+__global__ void k_keys(long long n, const Rec48* __restrict__ r, int low, const unsigned* __restrict__ idx, unsigned long long* key,
+                       unsigned* out_idx)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    hi[i] = r[i].hi;
-    lo[i] = r[i].lo;
-    idx[i] = (int)i;
+    const unsigned j = idx ? idx[i] : (unsigned)i;
+    key[i] = low ? r[j].lo : r[j].hi;
+    if (!idx) out_idx[i] = j;
 }
-__device__ __forceinline__ unsigned digit(const unsigned long long* hi, const unsigned long long* lo, long long i, int pass)
+// the coarsest and the finest level of the records
+__global__ void k_level_range(long long n, const Rec48* __restrict__ r, int* range)
 {
-    // passes 0-15 take lo's nibbles from the lowest, 16-31 hi's
-    const unsigned long long w = (pass < 16) ? lo[i] : hi[i];
-    return (unsigned)((w >> (4 * (pass & 15))) & 15ull);
-}
-__global__ void k_hist(long long n, const unsigned long long* __restrict__ hi, const unsigned long long* __restrict__ lo,
-                       int pass, int* hist, long long ntiles)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntiles) return;
-    int h[16];
-    for (int d = 0; d < 16; ++d) h[d] = 0;
-    const long long e = min(n, (t + 1) * kTile);
-    for (long long i = t * kTile; i < e; ++i) ++h[digit(hi, lo, i, pass)];
-    for (int d = 0; d < 16; ++d) hist[d * ntiles + t] = h[d];
-}
-__global__ void k_scatter(long long n, const unsigned long long* __restrict__ hi, const unsigned long long* __restrict__ lo,
-                          const int* __restrict__ idx, int pass, const int* __restrict__ off, long long ntiles,
-                          unsigned long long* hi2, unsigned long long* lo2, int* idx2)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntiles) return;
-    int o[16];
-    for (int d = 0; d < 16; ++d) o[d] = off[d * ntiles + t];
-    const long long e = min(n, (t + 1) * kTile);
-    for (long long i = t * kTile; i < e; ++i) {
-        const int j = o[digit(hi, lo, i, pass)]++;
-        hi2[j] = hi[i];
-        lo2[j] = lo[i];
-        idx2[j] = idx[i];
+    int lo = 64, hi = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int L = r[i].pad;
+        lo = min(lo, L);
+        hi = max(hi, L);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(range, lo);
+        atomicMax(range + 1, hi);
     }
 }
-__global__ void k_gather(long long n, const Rec48* __restrict__ in, const int* __restrict__ idx, Rec48* out)
+// the positions of the set flags, from their exclusive scan
+__global__ void k_flagged(long long n, const int* __restrict__ scan, int* list)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && scan[i + 1] > scan[i]) list[scan[i]] = (int)i;
+}
+__global__ void k_gather(long long n, const Rec48* __restrict__ in, const unsigned* __restrict__ idx, Rec48* out)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = in[idx[i]];
@@ -669,29 +660,28 @@ __device__ __forceinline__ float interpolate2(float x0, const double* x, const d
 // snapping.  The cells' scale factors as sortable 32-bit keys (non-negative
 // floats order as their bit patterns); the values the reference drops from its
 // table (sign bit set, or not normal) get 0xffffffff and sort last.
-__global__ void k_a_keys(long long n, const Rec48* __restrict__ r, unsigned long long* hi, unsigned long long* lo, int* idx)
+__global__ void k_a_keys(long long n, const Rec48* __restrict__ r, unsigned* key, unsigned* idx)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float a = r[i].a;
-    hi[i] = 0ull;
-    lo[i] = (!signbit(a) && normal_f(a)) ? (unsigned long long)__float_as_uint(a) : 0xffffffffull;
-    idx[i] = (int)i;
+    key[i] = (!signbit(a) && normal_f(a)) ? __float_as_uint(a) : 0xffffffffu;
+    idx[i] = (unsigned)i;
 }
 
 // the first of each run of equal sorted keys, the dropped values excluded
-__global__ void k_a_unique(long long n, const unsigned long long* __restrict__ lo, int* flag)
+__global__ void k_a_unique(long long n, const unsigned* __restrict__ key, int* flag)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    flag[i] = (lo[i] != 0xffffffffull && (i == 0 || lo[i] != lo[i - 1])) ? 1 : 0;
+    flag[i] = (key[i] != 0xffffffffu && (i == 0 || key[i] != key[i - 1])) ? 1 : 0;
 }
 
-__global__ void k_a_select(long long n, const unsigned long long* __restrict__ lo, const int* __restrict__ scan, float* table)
+__global__ void k_a_select(long long n, const unsigned* __restrict__ key, const int* __restrict__ scan, float* table)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (scan[i + 1] > scan[i]) table[scan[i]] = __uint_as_float((unsigned)lo[i]);
+    if (scan[i + 1] > scan[i]) table[scan[i]] = __uint_as_float(key[i]);
 }
 
 // each cell's a becomes the table's value below it, *(lower_bound(a) - 1);
@@ -730,20 +720,39 @@ using namespace mpf::build;
 namespace {
 int fail(int code, const std::string& m) { return mpf_internal_set_error(code, m.c_str()); }
 
+// Device scratch of one call: pieces of a few large blocks (an allocation and
+// its release cost about 100 us each), freed when the call ends.
 struct Arena {
-    std::vector<void*> ptrs;
+    std::vector<void*> blocks;
+    char* at = nullptr;
+    size_t left = 0;
     cudaError_t err = cudaSuccess;
+    // room for at least `bytes` more
+    void reserve(size_t bytes)
+    {
+        if (err != cudaSuccess || bytes <= left) return;
+        void* p = nullptr;
+        err = cudaMalloc(&p, bytes);
+        if (err != cudaSuccess) return;
+        blocks.push_back(p);
+        at = (char*)p;
+        left = bytes;
+    }
     template <class T>
     T* get(size_t count)
     {
-        void* p = nullptr;
-        if (err == cudaSuccess && count) err = cudaMalloc(&p, count * sizeof(T));
-        if (p) ptrs.push_back(p);
-        return (T*)p;
+        const size_t bytes = (count * sizeof(T) + 255) / 256 * 256;
+        if (bytes == 0) return nullptr;
+        reserve(bytes);
+        if (err != cudaSuccess) return nullptr;
+        T* const p = (T*)at;
+        at += bytes;
+        left -= bytes;
+        return p;
     }
     ~Arena()
     {
-        for (void* p : ptrs) cudaFree(p);
+        for (void* p : blocks) cudaFree(p);
     }
 };
 
@@ -782,25 +791,27 @@ long long compact(Arena& A, const Rec48* in, long long n, int* flag, Rec48* out,
     return total;
 }
 
-// sort n records by key (stable) into out
-void sort_records(Arena& A, const Rec48* in, long long n, Rec48* out, cudaStream_t s)
+// sort n records by key (stable) into out; nmax: their finest level.  A level's
+// key digit is 4 bits from the top, so two levels are one 8-bit digit and only
+// the levels that occur are sorted: 6 passes for levels to 12, not 32 nibbles.
+void sort_records(Arena& A, const Rec48* in, long long n, Rec48* out, int nmax, cudaStream_t s)
 {
-    unsigned long long *hi = A.get<unsigned long long>(n), *lo = A.get<unsigned long long>(n);
-    unsigned long long *hi2 = A.get<unsigned long long>(n), *lo2 = A.get<unsigned long long>(n);
-    int *idx = A.get<int>(n), *idx2 = A.get<int>(n);
-    const long long ntiles = (n + kTile - 1) / kTile;
-    int* hist = A.get<int>((size_t)16 * ntiles + 1);
+    unsigned long long *k1 = A.get<unsigned long long>(n), *k2 = A.get<unsigned long long>(n);
+    unsigned *p1 = A.get<unsigned>(n), *p2 = A.get<unsigned>(n);
+    int* scratch = A.get<int>(radix_scratch(n));
     if (A.err != cudaSuccess) return;
-    k_keys<<<blk(n, 256), 256, 0, s>>>(n, in, hi, lo, idx);
-    for (int pass = 0; pass < 32; ++pass) {
-        k_hist<<<blk(ntiles, 128), 128, 0, s>>>(n, hi, lo, pass, hist, ntiles);
-        exclusive_scan(hist, 16 * ntiles, s);
-        k_scatter<<<blk(ntiles, 128), 128, 0, s>>>(n, hi, lo, idx, pass, hist, ntiles, hi2, lo2, idx2);
-        std::swap(hi, hi2);
-        std::swap(lo, lo2);
-        std::swap(idx, idx2);
+    bool first = true;
+    for (int low = (nmax > 16) ? 1 : 0; low >= 0; --low) {
+        const int levels = low ? nmax - 16 : std::min(nmax, 16);
+        k_keys<<<blk(n, 256), 256, 0, s>>>(n, in, low, first ? nullptr : p1, k1, p1);
+        first = false;
+        for (int q = (levels + 1) / 2; q > 0; --q) {
+            radix_pass(n, k1, p1, k2, p2, 64 - 8 * q, scratch, s);
+            std::swap(k1, k2);
+            std::swap(p1, p2);
+        }
     }
-    k_gather<<<blk(n, 256), 256, 0, s>>>(n, in, idx, out);
+    k_gather<<<blk(n, 256), 256, 0, s>>>(n, in, p1, out);
 }
 
 // Input::correct's acorrection over the n records of r as the container
@@ -813,26 +824,21 @@ cudaError_t acorrect(Arena& A, Rec48* r, long long n, double* amin, cudaStream_t
 {
     if (n <= 0) return cudaSuccess;
     // the table of the cells' distinct scale factors, sorted on the device
-    unsigned long long *hi = A.get<unsigned long long>(n), *lo = A.get<unsigned long long>(n);
-    unsigned long long *hi2 = A.get<unsigned long long>(n), *lo2 = A.get<unsigned long long>(n);
-    int *idx = A.get<int>(n), *idx2 = A.get<int>(n), *uflag = A.get<int>(n + 1);
+    unsigned *k1 = A.get<unsigned>(n), *k2 = A.get<unsigned>(n), *p1 = A.get<unsigned>(n), *p2 = A.get<unsigned>(n);
+    int* uflag = A.get<int>(n + 1);
     float* dtable = A.get<float>(n + 1);
-    const long long ntiles = (n + kTile - 1) / kTile;
-    int* hist = A.get<int>((size_t)16 * ntiles + 1);
+    int* scratch = A.get<int>(radix_scratch(n));
     if (A.err != cudaSuccess) return A.err;
-    k_a_keys<<<blk(n, 256), 256, 0, s>>>(n, r, hi, lo, idx);
-    for (int pass = 0; pass < 8; ++pass) {
-        k_hist<<<blk(ntiles, 128), 128, 0, s>>>(n, hi, lo, pass, hist, ntiles);
-        exclusive_scan(hist, 16 * ntiles, s);
-        k_scatter<<<blk(ntiles, 128), 128, 0, s>>>(n, hi, lo, idx, pass, hist, ntiles, hi2, lo2, idx2);
-        std::swap(hi, hi2);
-        std::swap(lo, lo2);
-        std::swap(idx, idx2);
+    k_a_keys<<<blk(n, 256), 256, 0, s>>>(n, r, k1, p1);
+    for (int shift = 0; shift < 32; shift += 8) {
+        radix_pass(n, k1, p1, k2, p2, shift, scratch, s);
+        std::swap(k1, k2);
+        std::swap(p1, p2);
     }
-    k_a_unique<<<blk(n, 256), 256, 0, s>>>(n, lo, uflag);
+    k_a_unique<<<blk(n, 256), 256, 0, s>>>(n, k1, uflag);
     cudaMemsetAsync(uflag + n, 0, sizeof(int), s);
     const long long asize = exclusive_scan(uflag, n + 1, s);
-    k_a_select<<<blk(n, 256), 256, 0, s>>>(n, lo, uflag, dtable);
+    k_a_select<<<blk(n, 256), 256, 0, s>>>(n, k1, uflag, dtable);
     std::vector<float> table((size_t)asize);
     cudaError_t e = cudaSuccess;
     if (asize > 0) e = cudaMemcpy(table.data(), dtable, (size_t)asize * sizeof(float), cudaMemcpyDeviceToHost);
@@ -855,9 +861,9 @@ cudaError_t acorrect(Arena& A, Rec48* r, long long n, double* amin, cudaStream_t
 }
 
 // SimpleHyperOctree::update on device records: sort, collapse, compact
-long long update(Arena& A, Rec48* r, long long n, Rec48* tmp, int* flag, cudaStream_t s)
+long long update(Arena& A, Rec48* r, long long n, Rec48* tmp, int* flag, int nmax, cudaStream_t s)
 {
-    sort_records(A, r, n, tmp, s);
+    sort_records(A, r, n, tmp, nmax, s);
     if (A.err != cudaSuccess) return -1;
     k_collapse<<<blk(n, 256), 256, 0, s>>>(n, tmp, flag);
     return compact(A, tmp, n, flag, r, s);
@@ -924,6 +930,8 @@ extern "C" int mpf_cells_build(const float* rows, int64_t n, const mpf_cells_par
     G.mpc = cp->mpc;
     cudaStream_t s = 0;
     Arena A;
+    // rows, two copies of the records, flags and the sort's pairs
+    A.reserve((size_t)n * (40 + 2 * sizeof(Rec48) + 4 + 24 + 8) + radix_scratch(n) * 4 + 16 * 256);
     float* drows = A.get<float>((size_t)n * 10);
     Rec48 *r0 = A.get<Rec48>(n), *r1 = A.get<Rec48>(n);
     int* flag = A.get<int>(n + 1);
@@ -944,17 +952,17 @@ extern "C" int mpf_cells_build(const float* rows, int64_t n, const mpf_cells_par
     }
     // sistemize, dphidt = 0, update
     k_sistemize<<<blk(m, 256), 256, 0, s>>>(m, r1, G);
-    m = update(A, r1, m, r0, flag, s);
+    int* drange = A.get<int>(2);
+    int range[2] = {64, 0};
+    if (A.err != cudaSuccess) return fail(MPF_OUT_OF_MEMORY, "mpf_cells_build: device memory");
+    e = cudaMemcpyAsync(drange, range, sizeof(range), cudaMemcpyHostToDevice, s);
+    k_level_range<<<std::min(blk(m, 256), 1216u), 256, 0, s>>>(m, r1, drange);
+    if (e == cudaSuccess) e = cudaMemcpy(range, drange, sizeof(range), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return fail(MPF_CUDA_ERROR, std::string("mpf_cells_build: ") + cudaGetErrorString(e));
+    const int ncoarse = range[0], nmax = std::min(range[1], kMaxLevel);
+    m = update(A, r1, m, r0, flag, nmax, s);
     if (A.err != cudaSuccess || m < 0) return fail(MPF_OUT_OF_MEMORY, "mpf_cells_build: device memory");
     // Input::correct
-    std::vector<Rec48> h((size_t)m);
-    e = cudaMemcpy(h.data(), r1, (size_t)m * sizeof(Rec48), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return fail(MPF_CUDA_ERROR, std::string("mpf_cells_build: ") + cudaGetErrorString(e));
-    int ncoarse = 64, nmax = 0;
-    for (const Rec48& x : h) {
-        ncoarse = std::min(ncoarse, x.pad);
-        nmax = std::max(nmax, x.pad);
-    }
     if (cp->coarsecorrection) {
         float* rho0 = A.get<float>(m);
         if (A.err != cudaSuccess) return fail(MPF_OUT_OF_MEMORY, "mpf_cells_build: device memory");
@@ -988,18 +996,18 @@ extern "C" int mpf_cells_build(const float* rows, int64_t n, const mpf_cells_par
         ninc = exclusive_scan(flag, m + 1, s);
     }
     if (ninc > 0) {
+        // the list, the records and their copy with the children, flags, the
+        // children's waves and the final update's sort
+        A.reserve((size_t)(m + 8 * ninc) * (2 * sizeof(Rec48) + 4 + 24) + (size_t)ninc * 36 + radix_scratch(m + 8 * ninc) * 4 +
+                  (size_t)std::max(max_waves, 1) * 4 + 16 * 256);
         int* list = A.get<int>(ninc);
         Rec48* grown = A.get<Rec48>(m + 8 * ninc);
         Rec48* tmp = A.get<Rec48>(m + 8 * ninc);
         int* flag2 = A.get<int>(m + 8 * ninc + 1);
         if (A.err != cudaSuccess) return fail(MPF_OUT_OF_MEMORY, "mpf_cells_build: device memory");
         // the list of incomplete cells, in key order
-        std::vector<int> hflag((size_t)m + 1), hl;
-        cudaMemcpy(hflag.data(), flag, (size_t)(m + 1) * sizeof(int), cudaMemcpyDeviceToHost);
-        for (long long i = 0; i < m; ++i)
-            if (hflag[i + 1] > hflag[i]) hl.push_back((int)i);
-        cudaMemcpy(list, hl.data(), hl.size() * sizeof(int), cudaMemcpyHostToDevice);
-        cudaMemcpy(grown, r1, (size_t)m * sizeof(Rec48), cudaMemcpyDeviceToDevice);
+        k_flagged<<<blk(m, 256), 256, 0, s>>>(m, flag, list);
+        cudaMemcpyAsync(grown, r1, (size_t)m * sizeof(Rec48), cudaMemcpyDeviceToDevice, s);
         const long long nch = 8 * ninc;
         int* done = A.get<int>(nch);
         int* pending = A.get<int>(std::max(max_waves, 1));
@@ -1024,7 +1032,7 @@ extern "C" int mpf_cells_build(const float* rows, int64_t n, const mpf_cells_par
         // acorrection runs on the container with its appended children, before the final update
         if (cp->acorrection && (e = acorrect(A, grown, m + 8 * ninc, cp->amin, s)) != cudaSuccess)
             return fail(MPF_CUDA_ERROR, std::string("mpf_cells_build: ") + cudaGetErrorString(e));
-        m = update(A, grown, m + 8 * ninc, tmp, flag2, s);
+        m = update(A, grown, m + 8 * ninc, tmp, flag2, nmax, s);   // a child is no finer than a descendant that is there
         if (A.err != cudaSuccess || m < 0) return fail(MPF_OUT_OF_MEMORY, "mpf_cells_build: device memory");
         r1 = grown;
     } else if (cp->correction && cp->acorrection && (e = acorrect(A, r1, m, cp->amin, s)) != cudaSuccess) {

@@ -54,6 +54,9 @@ namespace mpf {
 
 // exclusive scan of n int32 values in place on `stream`; returns the total
 int64_t exclusive_scan(int* d, int64_t n, cudaStream_t stream);
+// the same without the total and without waiting; tmp: scan_scratch(n) ints
+size_t scan_scratch(int64_t n);
+void exclusive_scan_async(int* d, int64_t n, int* tmp, cudaStream_t stream);
 
 template <bool EXACT>
 cudaError_t launch_propagate(const DevTree& T, const DevCosmo& C, const PropParams& P, const double* d_launch, long long n,

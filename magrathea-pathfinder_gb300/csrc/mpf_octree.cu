@@ -276,6 +276,27 @@ int64_t exclusive_scan(int* d, int64_t n, cudaStream_t stream)
     return total;
 }
 
+size_t scan_scratch(int64_t n)
+{
+    size_t t = 0;
+    do {
+        n = (n + kScanBlock - 1) / kScanBlock;
+        t += (size_t)n;
+    } while (n > 1);
+    return t;
+}
+
+void exclusive_scan_async(int* d, int64_t n, int* tmp, cudaStream_t stream)
+{
+    if (n <= 0) return;
+    const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
+    k_scan_block<<<(unsigned)nb, kScanBlock, 0, stream>>>(d, n, tmp);
+    if (nb > 1) {
+        exclusive_scan_async(tmp, nb, tmp + nb, stream);
+        k_scan_add<<<(unsigned)nb, kScanBlock, 0, stream>>>(d, n, tmp);
+    }
+}
+
 }  // namespace mpf
 
 using namespace mpf;

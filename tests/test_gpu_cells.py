@@ -182,3 +182,44 @@ def test_rotated_build_equals_reference(gpu_lib, pkg):
     np.testing.assert_array_equal(got["lo"], ref["lo"])
     for name in ("dphidt", "a", "dphidx", "dphidy", "dphidz", "phi", "rho"):
         np.testing.assert_array_equal(got[name][:-1].view(np.uint32), ref[name][:-1].view(np.uint32), err_msg=name)
+
+
+@pytest.mark.parametrize("depth", [12, 16, 17, 21])
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 9000])
+def test_key_sort_matches_oracle(gpu_lib, pkg, oracle_mod, synth, depth, n):
+    """The sort of the keys (8-bit digits over the levels that occur, the low
+    half of the key only below level 16; tiles of 2048 pairs): n rows in
+    random order of a base grid with one chain of octs down to level `depth`
+    and a quarter of the rows given twice, against the oracle's build."""
+    g = load_golden("cells")
+    rng = np.random.default_rng(depth)
+    spec = synth.OctreeSpec(base_level=8, box_cells=64, lbox=2048.0, half_y=5.0, half_z=5.0, chi_max=900.0, halos=0, max_level=8,
+                            seed=3)
+    base = synth.cells_ramses(synth.make_octree(spec), spec).astype(np.float32)
+    point = np.array([0.21317, 0.00391, -0.00713])
+    chain = []
+    for L in range(9, depth + 1):
+        size = 4.0 / 2 ** L
+        oct0 = np.floor((point + 2.0) / (2 * size)) * 2 * size - 2.0
+        for s in range(8):
+            r = base[rng.integers(base.shape[0])].copy()
+            r[0] = L - 2
+            r[1:4] = oct0 + size * (np.array([s & 1, (s >> 1) & 1, s >> 2]) + 0.5)
+            chain.append(r)
+    rows = np.concatenate([np.array(chain, dtype=np.float32), base])
+    again = rows[rng.random(rows.shape[0]) < 0.25].copy()
+    again[:, 9] *= np.float32(1.001)
+    again[:, 5] *= np.float32(1.01)
+    rows = np.concatenate([rows, again])
+    rows = np.concatenate([rows[:len(chain)], rows[len(chain):][rng.permutation(rows.shape[0] - len(chain))]])[:n]
+    rows = rows[rng.permutation(rows.shape[0])]
+    cone7 = np.array([0.0, 0.0, 0.0, 0.5, 0.0, 0.0, np.radians(8.0)])
+    sphere4 = np.array([0.0, 0.0, 0.0, 1.0 / 32.0])
+    ref, _, info = oracle_mod.cells_build(rows, {"t": g["cosmo_t"], "a": g["cosmo_a"], "dadt": g["cosmo_dadt"]}, cone7, sphere4,
+                                          spec.cosmo.h, spec.lbox, float(g["mpc"]), completion_waves=32)
+    cos = pkg.Cosmology(g["cosmo_t"], g["cosmo_a"], g["cosmo_dadt"], g["cosmo_d2adt2"])
+    rec = pkg.cells_build(rows, cos, cone7[:3], cone7[3:6], cone7[6], sphere4[:3], sphere4[3], spec.cosmo.h,
+                          spec.cosmo.omega_m, spec.lbox, float(g["mpc"]))
+    assert pkg.cells_completion_info() == info
+    cos.close()
+    np.testing.assert_array_equal(rec, ref)
