@@ -170,3 +170,26 @@ def test_removing_the_field_restores_the_plain_build(gpu_lib, pkg, amr, cosmo):
     np.testing.assert_array_equal(s, g["ref_steps_o2"])
     np.testing.assert_array_equal(f.view(np.uint64), g["ref_final_o2"].view(np.uint64))
     tree.close()
+
+
+@pytest.mark.parametrize("scheme", ["cic", "tsc"])
+@pytest.mark.parametrize("n", [1, 75, 2048, 2049, 30000])
+def test_deposit_matches_oracle_at_tile_edges(gpu_lib, pkg, oracle_mod, synth, amr, scheme, n):
+    """The pair sort's tiles, the four-at-a-time run sums and the vertex cells
+    read from the stencil records against the C oracle, bit for bit: n
+    particles, a third of them in one place (one long run a cell), some on cell
+    faces, some outside the cone's cells."""
+    rng = np.random.default_rng(n)
+    pos, pv = synth.velocity_particles(amr["records"], n, seed=n)
+    pos[::3] = pos[0] + rng.uniform(-1e-4, 1e-4, pos[::3].shape).astype(np.float32)
+    pos[1::7] = np.round(pos[1::7] * 256) / 256
+    pos[2::11] = rng.uniform(-1.9, 1.9, pos[2::11].shape)
+    tree = pkg.Octree.from_records(amr["records"])
+    tree.deposit_velocity(pos, pv, scheme)
+    v, rho = tree.velocity()
+    tree.close()
+    O = oracle_mod.Oracle(amr["records"], {"t": amr["cosmo_t"], "a": amr["cosmo_a"], "dadt": amr["cosmo_dadt"]},
+                          float(amr["cosmo_length"]))
+    ov, orho = O.deposit_velocity(pos, pv, scheme)
+    np.testing.assert_array_equal(rho.view(np.uint32), np.asarray(orho, dtype=np.float32).view(np.uint32))
+    np.testing.assert_array_equal(v.view(np.uint32), np.asarray(ov, dtype=np.float32).view(np.uint32))
