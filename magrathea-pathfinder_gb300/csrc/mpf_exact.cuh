@@ -7,37 +7,20 @@
 // sub-partition for a warp's add, multiply, fused multiply-add, compare or
 // conversion alike, however many of its lanes are active.  A
 // field's multiply-accumulate is (float)((double)acc + (double)v * w): two
-// operations and three conversions.  The conversions are done on the integer
-// bits here, weights and vertex coordinates once per axis instead of once per
-// cell, the field at a step's start is the one already read after the step
-// before it, and a point's cell is looked for around the last one's.  4099
-// rays of 277 steps on a refined cone (TSC, Jacobian): 202 ms -> 66 ms, the
-// FP64 pipe busy 71 % of the time.
+// operations and three conversions.  The conversions, products with powers of
+// two, coordinates and table lookups are done on the integer bits here,
+// weights and vertex coordinates once per axis instead of once per cell, the
+// divisions by the box length by its reciprocal and two residuals, the record
+// fields that only a photon record reports at the ray's end; the field at a
+// step's start is the one already read after the step before it, and a point's
+// cell is looked for around the last one's.  4099 rays of 277 steps on a
+// refined cone (TSC, Jacobian): 202 ms -> 46 ms, the FP64 pipe busy 63 % of the
+// time.
 #pragma once
+#include "mpf_fp64.cuh"
 #include "mpf_propagate.cuh"
 
 namespace mpf {
-
-// (double)v on the integer bits for normal numbers
-__device__ __forceinline__ double wide(float v)
-{
-    const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
-    if (a - 0x00800000u < 0x7f000000u)
-        return __hiloint2double((int)(((a >> 3) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
-    return (double)v;
-}
-
-// (double)(float)d on the integer bits where the result is a normal float
-// below 2^127: round to nearest even at bit 29
-__device__ __forceinline__ double round32(double d)
-{
-    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-    if ((hi & 0x7fffffffu) - 0x38100000u < 0x47e00000u - 0x38100000u) {
-        const unsigned l2 = lo + 0x0fffffffu + ((lo >> 29) & 1u);
-        return __hiloint2double((int)(hi + (l2 < lo ? 1u : 0u)), (int)(l2 & 0xe0000000u));
-    }
-    return (double)__double2float_rn(d);
-}
 
 // acc += v * w with the reference's rounding, the accumulator a float held in
 // a double: (float)((double)acc + (double)v * w)
@@ -87,6 +70,39 @@ struct ExactAcc {
         return Field7{(float)rho, (float)phi, (float)dx, (float)dy, (float)dz, (float)a, (float)dt};
     }
 };
+
+// axis_coord(L, x), its product with the power of two and its truncation on
+// the integer bits where x lies in the domain
+__device__ __forceinline__ uint64_t axis_coord_bits(int L, double x)
+{
+    const double u = __dadd_rn(x, (double)kExtent / 2.0);
+    const unsigned hi = (unsigned)__double2hiint(u);
+    // 2^-512 <= u < 4
+    if (hi - 0x1ff00000u < 0x40100000u - 0x1ff00000u) {
+        const int drop = 52 - ((int)(hi >> 20) - 1023) - (L - kLevelShift);
+        const uint64_t m = ((uint64_t)__double_as_longlong(u) & 0xfffffffffffffull) | 0x10000000000000ull;
+        return (drop < 53) ? m >> drop : 0ull;
+    }
+    return axis_coord(L, x);
+}
+
+// coord_center(L, c) for c < 2^32: c + 1/2 from the bits of 2^52 + c, the rest
+// exact as there
+__device__ __forceinline__ double coord_center_bits(int L, uint64_t c)
+{
+    const double v = __dsub_rn(__hiloint2double(0x43300000, (int)(uint32_t)c), 4503599627370495.5);
+    return __dadd_rn(times_pow2(v, kLevelShift - L), -(double)kExtent / 2.0);
+}
+
+// a / b for a divisor with y = 1 / b rounded to nearest, correctly rounded
+// where nothing over- or underflows (Markstein, IBM J. Res. Dev. 34, 1990: a
+// quotient within one ulp and the residual of a fused multiply-add)
+__device__ __forceinline__ double divide_by(double a, double b, double y)
+{
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
 
 // A cell near the next point looked for, and its integer coordinates.
 struct Hint {
@@ -172,7 +188,7 @@ __device__ Field7 cic_exact(const DevTree& T, double x, double y, double z, Hint
 {
     ExactAcc<F, V> res;
     res.reset();
-    const uint64_t c32[3] = {axis_coord(kMaxLevel, x), axis_coord(kMaxLevel, y), axis_coord(kMaxLevel, z)};
+    const uint64_t c32[3] = {axis_coord_bits(kMaxLevel, x), axis_coord_bits(kMaxLevel, y), axis_coord_bits(kMaxLevel, z)};
     const Found f0 = locate_near32(T, c32, hint);
     if (f0.cell < 0) return res.field(vv);
     int ilvl = f0.level, lvl = ilvl;
@@ -182,7 +198,6 @@ __device__ Field7 cic_exact(const DevTree& T, double x, double y, double z, Hint
         if (lvl < ilvl) centre = ancestor_cell(T, centre, ilvl, lvl);
         ilvl = lvl;
         const double half = half_cell(ilvl);
-        const double inv = pow2(ilvl - kLevelShift);   // 1 / (half + half), exact
         const uint64_t m = (1ull << ilvl) - 1ull;
         uint64_t cc[3], k[3][2];
         double w[3][2];   // by the vertex's bit
@@ -194,13 +209,14 @@ __device__ Field7 cic_exact(const DevTree& T, double x, double y, double z, Hint
             cc[d] = c32[d] >> (kMaxLevel - ilvl);
             const int s = (ilvl < kMaxLevel) ? (int)((c32[d] >> (kMaxLevel - ilvl - 1)) & 1ull) : 0;
             site |= s << d;
-            const double dist = fabs(__dmul_rn(__dsub_rn(coord_center(ilvl, cc[d]), pt[d]), inv));
+            // over the cell size, a power of two
+            const double dist = fabs(times_pow2(__dsub_rn(coord_center_bits(ilvl, cc[d]), pt[d]), ilvl - kLevelShift));
             // the neighbour on the point's side weighs dist, the centre cell 1 - dist
             const double rest = __dsub_rn(1.0, dist);
             w[d][0] = s ? rest : dist;
             w[d][1] = s ? dist : rest;
-            k[d][0] = axis_coord(ilvl, __dsub_rn(__dadd_rn(pt[d], 0.0), half));
-            k[d][1] = axis_coord(ilvl, __dadd_rn(pt[d], half));
+            k[d][0] = axis_coord_bits(ilvl, __dsub_rn(pt[d], half));
+            k[d][1] = axis_coord_bits(ilvl, __dadd_rn(pt[d], half));
             base[d] = s - 1;
             near = near && k[d][0] == ((cc[d] + (uint64_t)(int64_t)(s - 1)) & m) && k[d][1] == ((cc[d] + (uint64_t)s) & m);
         }
@@ -231,12 +247,15 @@ __device__ Field7 cic_exact(const DevTree& T, double x, double y, double z, Hint
     return res.field(vv);
 }
 
+// the reference's a * 0.5 * (1.5 - d) * (1.5 - d) + (1 - a) * (0.75 - d * d),
+// left to right, for a = 0 or 1: the other term is an exact zero
 __device__ __forceinline__ double tsc_w1(int a, double d)
 {
-    // (a*0.5*(1.5-d)*(1.5-d) + (1-a)*(0.75-d*d)), left to right, no contraction
-    const double t1 = __dmul_rn(__dmul_rn(__dmul_rn((double)a, 0.5), __dsub_rn(1.5, d)), __dsub_rn(1.5, d));
-    const double t2 = __dmul_rn((double)(1 - a), __dsub_rn(0.75, __dmul_rn(d, d)));
-    return __dadd_rn(t1, t2);
+    if (a) {
+        const double e = __dsub_rn(1.5, d);
+        return __dmul_rn(times_pow2(e, -1), e);
+    }
+    return __dsub_rn(0.75, __dmul_rn(d, d));
 }
 
 // Triangular-shaped cloud (simplehyperoctree.h:1479-1644): quadratic weights
@@ -249,7 +268,7 @@ __device__ Field7 tsc_exact(const DevTree& T, double x, double y, double z, Hint
     if (x == 0.0 && y == 0.0 && z == 0.0) return cic_exact<F, V>(T, 0., 0., 0., hint, vv);
     ExactAcc<F, V> res;
     res.reset();
-    const uint64_t c32[3] = {axis_coord(kMaxLevel, x), axis_coord(kMaxLevel, y), axis_coord(kMaxLevel, z)};
+    const uint64_t c32[3] = {axis_coord_bits(kMaxLevel, x), axis_coord_bits(kMaxLevel, y), axis_coord_bits(kMaxLevel, z)};
     const Found f0 = locate_near32(T, c32, hint);
     if (f0.cell < 0) return res.field(vv);
     int ilvl = f0.level, lvl = ilvl;
@@ -258,8 +277,7 @@ __device__ Field7 tsc_exact(const DevTree& T, double x, double y, double z, Hint
     do {
         if (lvl < ilvl) centre = ancestor_cell(T, centre, ilvl, lvl);
         ilvl = lvl;
-        const double tw = __dmul_rn(2.0, half_cell(ilvl));
-        const double inv = pow2(ilvl - kLevelShift);   // 1 / tw, exact
+        const double tw = cell_extent(ilvl);
         const uint64_t m = (1ull << ilvl) - 1ull;
         uint64_t cc[3], k[3][3];
         double w[3][3];
@@ -267,13 +285,20 @@ __device__ Field7 tsc_exact(const DevTree& T, double x, double y, double z, Hint
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             cc[d] = c32[d] >> (kMaxLevel - ilvl);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                k[d][i] = axis_coord(ilvl, __dadd_rn(pt[d], __dmul_rn((double)(i - 1), tw)));
-                const double dist = fabs(__dmul_rn(__dsub_rn(coord_center(ilvl, k[d][i]), pt[d]), inv));
-                w[d][i] = tsc_w1(i != 1, dist);
-                near = near && k[d][i] == ((cc[d] + (uint64_t)(int64_t)(i - 1)) & m);
-            }
+            k[d][0] = axis_coord_bits(ilvl, __dsub_rn(pt[d], tw));
+            k[d][1] = cc[d];
+            k[d][2] = axis_coord_bits(ilvl, __dadd_rn(pt[d], tw));
+            const bool next = k[d][0] == ((cc[d] - 1ull) & m) && k[d][2] == ((cc[d] + 1ull) & m);
+            near = near && next;
+            // the vertices' cell centres, one cell apart in the usual case (exact)
+            const double c1 = coord_center_bits(ilvl, cc[d]);
+            const bool inside = next && cc[d] > 0ull && cc[d] < m;
+            const double c0 = inside ? __dsub_rn(c1, tw) : coord_center(ilvl, k[d][0]);
+            const double c2 = inside ? __dadd_rn(c1, tw) : coord_center(ilvl, k[d][2]);
+            // over the cell size, a power of two
+            w[d][0] = tsc_w1(1, fabs(times_pow2(__dsub_rn(c0, pt[d]), ilvl - kLevelShift)));
+            w[d][1] = tsc_w1(0, fabs(times_pow2(__dsub_rn(c1, pt[d]), ilvl - kLevelShift)));
+            w[d][2] = tsc_w1(1, fabs(times_pow2(__dsub_rn(c2, pt[d]), ilvl - kLevelShift)));
         }
         if (near) {
             // the vertices are the record's 27 cells in order
@@ -354,7 +379,7 @@ __device__ __forceinline__ Field7 field_vel_at(const DevTree& T, const PropParam
 __device__ __forceinline__ Found locate_at(const DevTree& T, const PropParams& P, double x, double y, double z, Hint& hint)
 {
     if (P.homogeneous == 1) return Found{0, P.hom_level};
-    const uint64_t c32[3] = {axis_coord(kMaxLevel, x), axis_coord(kMaxLevel, y), axis_coord(kMaxLevel, z)};
+    const uint64_t c32[3] = {axis_coord_bits(kMaxLevel, x), axis_coord_bits(kMaxLevel, y), axis_coord_bits(kMaxLevel, z)};
     return locate_near32(T, c32, hint);
 }
 
@@ -367,25 +392,41 @@ struct RaySet {
 
 __device__ __forceinline__ bool vel_zero(const float* v) { return v[0] == 0.f && v[1] == 0.f && v[2] == 0.f; }
 
-// geodesic RHS (integrator.h:409-445) from the field at the point
-__device__ __forceinline__ void rhs(const DevCosmo& C, const PropParams& P, const Field7& d, const double* in, double* out)
+// Utility::interpolate with the upper bound carried from call to call: a ray's
+// conformal time moves by less than a table interval between two calls
+__device__ __forceinline__ double interpolate_near(double x0, const double* __restrict__ x, const double* __restrict__ y, int n, int& first)
+{
+    while (first < n && !less64(x0, __ldg(x + first))) ++first;
+    while (first > 0 && less64(x0, __ldg(x + first - 1))) --first;
+    int i = first;
+    i += (n > 1) * ((i <= 0) - (i >= n));
+    if (n > 1) {
+        const double xi = __ldg(x + i), xm = __ldg(x + i - 1), yi = __ldg(y + i), ym = __ldg(y + i - 1);
+        return ym + ((yi - ym) * (x0 - xm) / (xi - xm));
+    }
+    return (n > 0) ? __ldg(y) : 0.0;
+}
+
+// geodesic RHS (integrator.h:409-445) from the field at the point; y = 1 /
+// scale rounded, first = the upper bound of the conformal time
+__device__ __forceinline__ void rhs(const DevCosmo& C, double scale, double y, const Field7& f, const double* in, int& first, double* out)
 {
     const double two = 2.0;
     const double c2 = kC * kC;
-    const double dphidl = (double)d.dt * in[5] + ((double)d.dx * in[6] + (double)d.dy * in[7] + (double)d.dz * in[8]);
-    const double dadt = interpolate(in[1], C.t, C.dadt, C.n);
-    const double scale = P.length;
+    const double dt = wide(f.dt), dx = wide(f.dx), dy = wide(f.dy), dz = wide(f.dz);
+    const double dphidl = dt * in[5] + (dx * in[6] + dy * in[7] + dz * in[8]);
+    const double dadt = interpolate_near(in[1], C.t, C.dadt, C.n, first);
     out[0] = in[5] * dadt;
     out[1] = in[5];
-    out[2] = in[6] / scale;
-    out[3] = in[7] / scale;
-    out[4] = in[8] / scale;
+    out[2] = divide_by(in[6], scale, y);
+    out[3] = divide_by(in[7], scale, y);
+    out[4] = divide_by(in[8], scale, y);
     const double hub = two * dadt / in[0] * in[5];
-    out[5] = -(hub * in[5]) - (two / c2 * in[5]) * (dphidl - (double)d.dt * in[5]);
+    out[5] = -(hub * in[5]) - (two / c2 * in[5]) * (dphidl - dt * in[5]);
     const double g = two / c2 * dphidl;
-    out[6] = -(hub * in[6]) + (g * in[6]) - (two * (double)d.dx * in[5] * in[5]);
-    out[7] = -(hub * in[7]) + (g * in[7]) - (two * (double)d.dy * in[5] * in[5]);
-    out[8] = -(hub * in[8]) + (g * in[8]) - (two * (double)d.dz * in[5] * in[5]);
+    out[6] = -(hub * in[6]) + (g * in[6]) - (two * dx * in[5] * in[5]);
+    out[7] = -(hub * in[7]) + (g * in[7]) - (two * dy * in[5] * in[5]);
+    out[8] = -(hub * in[8]) + (g * in[8]) - (two * dz * in[5] * in[5]);
 }
 
 __device__ __forceinline__ double plane_q(int kind, const Rec& r, const double* ki = nullptr)
@@ -447,16 +488,18 @@ __device__ void jac_point(const DevTree& T, const Rec& p, const Hint& at, double
     for (int q = 0; q < 6; ++q)
         for (int c = 0; c < 3; ++c) g[q][c] = R.points[3 * q + c];
     __syncwarp(R.mask);
-    const double phi = atan2(y, x);
-    const double theta = acos(z / r);
-    const double cp = cos(phi), sp = sin(phi), ct = cos(theta), st = sin(theta);
-    const double s2p = sin(2 * phi), s2t = sin(2 * theta);
-    const double dxxp = (double)(g[1][0] - g[0][0]) / dl;
-    const double dxyp = (double)(g[3][0] - g[2][0]) / dl;
-    const double dxzp = (double)(g[5][0] - g[4][0]) / dl;
-    const double dyyp = (double)(g[3][1] - g[2][1]) / dl;
-    const double dyzp = (double)(g[5][1] - g[4][1]) / dl;
-    const double dzzp = (double)(g[5][2] - g[4][2]) / dl;
+    // the direction's sines and cosines from its coordinates; 1 / dl is a power
+    // of two
+    const double rho = sqrt(x * x + y * y);
+    const double cp = (rho > 0.0) ? x / rho : 1.0, sp = (rho > 0.0) ? y / rho : 0.0, ct = z / r, st = rho / r;
+    const double s2p = 2.0 * sp * cp, s2t = 2.0 * st * ct;
+    const int e = (int)p.level - kLevelShift - 1;
+    const double dxxp = times_pow2(wide(g[1][0] - g[0][0]), e);
+    const double dxyp = times_pow2(wide(g[3][0] - g[2][0]), e);
+    const double dxzp = times_pow2(wide(g[5][0] - g[4][0]), e);
+    const double dyyp = times_pow2(wide(g[3][1] - g[2][1]), e);
+    const double dyzp = times_pow2(wide(g[5][1] - g[4][1]), e);
+    const double dzzp = times_pow2(wide(g[5][2] - g[4][2]), e);
     const double d1d1p = sp * sp * dxxp + cp * cp * dyyp - s2p * dxyp;
     const double d2d2p = cp * cp * ct * ct * dxxp + sp * sp * ct * ct * dyyp + st * st * dzzp + s2p * ct * ct * dxyp -
                          sp * s2t * dyzp - cp * s2t * dxzp;
@@ -555,29 +598,43 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
     Rec p = b;
     p.isw = zero; p.iswold = zero; p.lambda = zero; p.s = zero;
     double core[9], dc0[9], dc1[9], dc2[9], dc3[9];
+    const double inv_scale = __drcp_rn(scale);
+    int first = 0;   // upper bound of the ray's conformal time in the table
+    // the photon record's fields that no later step reads: formed for every
+    // point of a trajectory, else for the last one
+    double last_phi = b.phi, last_dl = one;
+    float last_dt = data.dt;
+    auto record_fields = [&](Rec& r) {
+        if (r.index == zero) return;
+        r.dphidl = (double)last_dt * r.k0 + (r.dx * r.k1 + r.dy * r.k2 + r.dz * r.k3);
+        r.lap = (r.phi - last_phi) / last_dl;
+        const double kk = r.k1 * r.k1 + r.k2 * r.k2 + r.k3 * r.k3;
+        r.ds2 = (r.a * r.a) * ((-c2 * (one + two * (r.phi / c2)) * r.k0 * r.k0) + ((one - two * (r.phi / c2)) * kk));
+        r.err = one - ((one - two * (r.phi / c2)) * kk) / (c2 * (one + two * (r.phi / c2)) * r.k0 * r.k0);
+    };
     while (!(is_empty(data) && vel_zero(vel))) {
         if (k >= P.max_steps) { status |= 1u; break; }
         const double bcore[9] = {b.a, b.t, b.x, b.y, b.z, b.k0, b.k1, b.k2, b.k3};
         p.index = b.index + one;
         // the field at b is the one read after the previous step
-        rhs(C, P, data, bcore, dc0);
+        rhs(C, scale, inv_scale, data, bcore, first, dc0);
 #pragma unroll
         for (int q = 0; q < 9; ++q) core[q] = bcore[q] + dl / two * dc0[q];
         {
             Hint h = hint;
-            rhs(C, P, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, dc1);
+            rhs(C, scale, inv_scale, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, first, dc1);
         }
 #pragma unroll
         for (int q = 0; q < 9; ++q) core[q] = bcore[q] + dl / two * dc1[q];
         {
             Hint h = hint;
-            rhs(C, P, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, dc2);
+            rhs(C, scale, inv_scale, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, first, dc2);
         }
 #pragma unroll
         for (int q = 0; q < 9; ++q) core[q] = bcore[q] + dl * dc2[q];
         {
             Hint h = hint;
-            rhs(C, P, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, dc3);
+            rhs(C, scale, inv_scale, field_at<kGradient4>(T, P, core[2], core[3], core[4], h), core, first, dc3);
         }
 #pragma unroll
         for (int q = 0; q < 9; ++q) core[q] = bcore[q] + (dl / six) * (dc0[q] + two * dc1[q] + two * dc2[q] + dc3[q]);
@@ -590,18 +647,12 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
             vel[0] = vel[1] = vel[2] = 0.f;
         }
         p.level = (loc.cell >= 0) ? (double)loc.level : 0.0;
-        p.ah = data.a;
-        p.rho = data.rho; p.phi = data.phi; p.dx = data.dx; p.dy = data.dy; p.dz = data.dz;
-        p.dt = -(double)data.dt;
-        p.dphidl = (double)data.dt * p.k0 + (p.dx * p.k1 + p.dy * p.k2 + p.dz * p.k3);
-        p.lap = ((double)data.phi - b.phi) / dl;
-        {
-            const double kk = p.k1 * p.k1 + p.k2 * p.k2 + p.k3 * p.k3;
-            p.ds2 = (p.a * p.a) * ((-c2 * (one + two * (p.phi / c2)) * p.k0 * p.k0) + ((one - two * (p.phi / c2)) * kk));
-            p.err = one - ((one - two * (p.phi / c2)) * kk) / (c2 * (one + two * (p.phi / c2)) * p.k0 * p.k0);
-        }
+        p.ah = wide(data.a);
+        p.rho = wide(data.rho); p.phi = wide(data.phi); p.dx = wide(data.dx); p.dy = wide(data.dy); p.dz = wide(data.dz);
+        p.dt = -wide(data.dt);
         p.isw += (b.dt + p.dt) * (p.t - b.t) / c2;
-        p.iswold -= 2 * (p.phi - b.phi) / c2 -
+        if (O.final_rec || traj)   // photon records only
+            p.iswold -= 2 * (p.phi - b.phi) / c2 -
                     ((b.dx + p.dx) * (p.x - b.x) * scale + (b.dy + p.dy) * (p.y - b.y) * scale + (b.dz + p.dz) * (p.z - b.z) * scale) / c2;
         p.chi = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
         p.lambda += dl;
@@ -613,7 +664,9 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
             p.red = a0 / p.a * (one + phi0c2 - p.phi / c2) - one;
         }
         bool appended = false;
+        double step = dl;
         if (!(is_empty(data) && vel_zero(vel))) {
+            step = dl;
             ratio = p.a * p.a * (scale / kC) / P.nsteps;
             dl = (loc.cell >= 0 ? cell_extent(loc.level) : 0.0) * ratio;
             appended = true;
@@ -621,6 +674,9 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
         if (appended) {
             // the new point p becomes trajectory[k+1]; b is trajectory[k]
             ++k;
+            last_phi = b.phi;
+            last_dl = step;
+            last_dt = data.dt;
             if (P.jacobian) {
                 double H[3];
                 jac_point(T, p, hint, p.chi - b.chi, H, R);
@@ -689,6 +745,7 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
             have_rmax = true;
             b = p;
             if (traj) {
+                record_fields(b);
                 if (k < O.traj_cap) write_rec(traj + k * kPhotonFields, b);
                 else status |= 8u;
             }
@@ -717,7 +774,10 @@ __device__ void propagate_one(const DevTree& T, const DevCosmo& C, const PropPar
     O.steps[i] = size;
     if (O.final_rec) {
         double* o = O.final_rec + i * kPhotonFields;
-        if (size == k + 1) write_rec(o, b);
+        if (size == k + 1) {
+            record_fields(b);
+            write_rec(o, b);
+        }
         else {
             // the popped point is not reported; the record before it is not kept,
             // so report zeros with the step count (only rays ending at z<0 or a<0)
