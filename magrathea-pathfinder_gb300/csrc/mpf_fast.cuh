@@ -921,6 +921,38 @@ __device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, dou
               cp * s2t * dxz;
 }
 
+// The surface record between two trajectory points (hmaps.h:612-676), the
+// Jacobian aside: out of line, a step crosses a surface once in a ray.
+struct SurfaceEnd {
+    double x, y, z, t, a, red, chi, lambda, s, isw, rho, phi, k0, k1, k2, k3;
+};
+static __device__ __noinline__ void write_surface(double* o, bool wide_record, double first, double f, SurfaceEnd b, SurfaceEnd p,
+                                                  double rmax)
+{
+    const double px = b.x * f + p.x * (1 - f), py = b.y * f + p.y * (1 - f), pz = b.z * f + p.z * (1 - f);
+    o[0] = first; o[1] = f; o[2] = px; o[3] = py; o[4] = pz; o[5] = sqrt(px * px + py * py + pz * pz);
+    o[6] = o[7] = o[8] = 0.0;
+    o[9] = b.t * f + p.t * (1 - f);
+    o[10] = b.a * f + p.a * (1 - f);
+    o[11] = b.red * f + p.red * (1 - f);
+    o[12] = b.chi * f + p.chi * (1 - f);
+    o[13] = b.lambda * f + p.lambda * (1 - f);
+    o[14] = b.s * f + p.s * (1 - f);
+    o[15] = b.isw * f + p.isw * (1 - f);
+    o[16] = b.rho * f + p.rho * (1 - f);
+    o[17] = b.phi * f + p.phi * (1 - f);
+    o[18] = rmax;
+    o[19] = 1.0;
+    if (wide_record) {
+        o[20] = b.k0 * f + p.k0 * (1 - f);
+        o[21] = b.k1 * f + p.k1 * (1 - f);
+        o[22] = b.k2 * f + p.k2 * (1 - f);
+        o[23] = b.k3 * f + p.k3 * (1 - f);
+    }
+}
+
+static __device__ __noinline__ double distance_of(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
+
 // a trajectory point's state and the field there
 struct RayPoint {
     double a, t, x, y, z, k0, k1, k2, k3, chi;
@@ -1015,11 +1047,15 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     auto red_above = [&](double a, float phi, double isw, double dop, double zref) -> bool {
         return a0 * zbracket(phi, isw, dop) > (1.0 + zref) * a;
     };
+    // the comoving distance is carried where each step reads it (the Jacobian,
+    // the stop at a radius, trajectories), else formed where a record does: its
+    // square root is a tenth of the FP64 operations of a CIC step
+    const bool want_chi = P.jacobian || skind == STOP_R || (WIDE && O.traj);
     // the point b as the reference's photon record
     auto full_point = [&]() -> FastRec {
         FastRec r;
         r.a = b.a; r.t = b.t; r.x = b.x; r.y = b.y; r.z = b.z; r.k0 = b.k0; r.k1 = b.k1; r.k2 = b.k2; r.k3 = b.k3;
-        r.phi = b.g.phi; r.chi = b.chi; r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw(); r.iswold = J.iswold();
+        r.phi = b.g.phi; r.chi = (want_chi || k == 0) ? b.chi : distance_of(b.x, b.y, b.z); r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw(); r.iswold = J.iswold();
         r.red = (k == 0) ? 0.0 : red_of(b.a, b.g.phi, r.isw, bdop);
         r.rho = b.g.rho; r.dx = b.g.dx; r.dy = b.g.dy; r.dz = b.g.dz; r.dt = bdt; r.ah = bah;
         r.level = (here.cell >= 0) ? here.level : 0;
@@ -1254,13 +1290,13 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         J.lambda() = p_lambda;
         if (O.final_rec || (WIDE && traj)) {   // reported by photon records only
             if (O.final_rec)
-                J.iswold() -= 2.0 * ((double)p.g.phi - (double)b.g.phi) * (1.0 / c2) -
-                              (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) * scale + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) * scale +
-                               ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z) * scale) * (1.0 / c2);
+                J.iswold() -= ((double)p.g.phi - (double)b.g.phi) * (2.0 * inv_c2) -
+                              (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) +
+                               ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z)) * (scale * inv_c2);
             J.last_dphi() = p.g.phi - b.g.phi;   // laplacian of the record, divided there
             J.last_dl() = dl;
         }
-        p.chi = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
+        if (want_chi) p.chi = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
         dl = (q.cell >= 0 ? cell_extent(q.level) : 0.0) * (p.a * p.a * ratio_k);
         ++k;
         // the surfaces the step crossed: everything but the Jacobian, from b and p
@@ -1287,32 +1323,18 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
             if (prow) {
                 if (!p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, pdop); p_red_known = true; }
                 const double b_red = (k == 1) ? 0.0 : red_of(b.a, b.g.phi, b_isw, bdop);
+                const double b_chi = want_chi ? b.chi : (k == 1) ? 0.0 : distance_of(b.x, b.y, b.z);
+                const double p_chi = want_chi ? p.chi : distance_of(p.x, p.y, p.z);
                 double* o = prow + j * rec_fields;
                 if (!kj && skind == STOP_REDSHIFT) q1 = p_red;
                 const double q0 = kj ? (b.x * kj[0] + b.y * kj[1] + b.z * kj[2])
                                 : (skind == STOP_R) ? b.chi : (skind == STOP_LAMBDA) ? b_lambda : (skind == STOP_T) ? b.t
                                 : (skind == STOP_A) ? b.a : (skind == STOP_S) ? b_s : b_red;
-                const double f = (q1 - ref) / (q1 - q0);
-                const double px = b.x * f + p.x * (1 - f), py = b.y * f + p.y * (1 - f), pz = b.z * f + p.z * (1 - f);
-                o[0] = (double)(k - 1); o[1] = f; o[2] = px; o[3] = py; o[4] = pz; o[5] = sqrt(px * px + py * py + pz * pz);
-                o[6] = o[7] = o[8] = 0.0;
-                o[9] = b.t * f + p.t * (1 - f);
-                o[10] = b.a * f + p.a * (1 - f);
-                o[11] = b_red * f + p_red * (1 - f);
-                o[12] = b.chi * f + p.chi * (1 - f);
-                o[13] = b_lambda * f + p_lambda * (1 - f);
-                o[14] = b_s * f + p_s * (1 - f);
-                o[15] = b_isw * f + p_isw * (1 - f);
-                o[16] = (double)b.g.rho * f + (double)p.g.rho * (1 - f);
-                o[17] = (double)b.g.phi * f + (double)p.g.phi * (1 - f);
-                o[18] = (k >= 2) ? (double)J.rmax() : 0.0;
-                o[19] = 1.0;
-                if (SRC || WIDE) {
-                    o[20] = b.k0 * f + p.k0 * (1 - f);
-                    o[21] = b.k1 * f + p.k1 * (1 - f);
-                    o[22] = b.k2 * f + p.k2 * (1 - f);
-                    o[23] = b.k3 * f + p.k3 * (1 - f);
-                }
+                const SurfaceEnd e0{b.x, b.y, b.z, b.t, b.a, b_red, b_chi, b_lambda, b_s, b_isw, (double)b.g.rho, (double)b.g.phi,
+                                    b.k0, b.k1, b.k2, b.k3};
+                const SurfaceEnd e1{p.x, p.y, p.z, p.t, p.a, p_red, p_chi, p_lambda, p_s, p_isw, (double)p.g.rho, (double)p.g.phi,
+                                    p.k0, p.k1, p.k2, p.k3};
+                write_surface(o, SRC || WIDE, (double)(k - 1), (q1 - ref) / (q1 - q0), e0, e1, (k >= 2) ? (double)J.rmax() : 0.0);
             }
         }
         // the largest density of the points before the new one
