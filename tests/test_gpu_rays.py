@@ -79,6 +79,30 @@ def test_batch_of_bundles_matches_oracle(rays_dev, pkg, oracle_mod, synth):
     assert (sizes > 0).sum() >= n // 2
 
 
+@pytest.mark.parametrize("capacity", [400, 1500])
+def test_central_points_come_back_over_several_copies(rays_dev, pkg, oracle_mod, synth, capacity):
+    """More points than one copy of the results holds, rejected bundles among
+    them: bundles over the whole batch against the C oracle, exact mode, and
+    nothing written behind a trajectory's end."""
+    g, tree, cos = rays_dev
+    n = 200
+    ph = np.resize(synth.photon_grid(15, 1.0, 1.0), (n, 6)).copy()
+    ph[1::7, 0] = 0.4                                    # leaves the box too soon: rejected
+    rot = np.linspace(0.0, 3.0, n)
+    kw = dict(nsteps=int(g["nsteps"]), order=1)
+    sizes, traj = pkg.rays_propagate(tree, cos, ph, float(g["cosmo_length"]), 2, np.radians(0.25), rotation=rot,
+                                     interpolation="r", exact=True, capacity=capacity, **kw)
+    assert sizes.max() * n * traj.shape[2] * 8 > 4 << 20 and (sizes == 0).any()
+    O = oracle_mod.Oracle(g["records"], {"t": g["cosmo_t"], "a": g["cosmo_a"], "dadt": g["cosmo_dadt"]},
+                          float(g["cosmo_length"]), nthreads=1)
+    for i in list(range(0, n, 17)) + [1, 8, n - 1]:
+        ref = O.propagate_bundle(ph[i], 2, np.radians(0.25), rot[i], "r", 0.0, **kw)
+        assert sizes[i] == ref.shape[0], i
+        np.testing.assert_array_equal(traj[i, :sizes[i]].view(np.uint64), ref.view(np.uint64))
+    for i in range(n):
+        assert not traj[i, sizes[i]:].any(), i
+
+
 def test_capacity_too_small_is_an_error(rays_dev, pkg):
     g, tree, cos = rays_dev
     with pytest.raises(pkg.MpfError):
