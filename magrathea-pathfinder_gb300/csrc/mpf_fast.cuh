@@ -1289,9 +1289,10 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         J.s() = p_s;
         J.lambda() = p_lambda;
         if (O.final_rec || (WIDE && traj)) {   // reported by photon records only
-            J.iswold() -= ((double)p.g.phi - (double)b.g.phi) * (2.0 * inv_c2) -
-                          (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) +
-                           ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z)) * (scale * inv_c2);
+            if (O.final_rec)
+                J.iswold() -= ((double)p.g.phi - (double)b.g.phi) * (2.0 * inv_c2) -
+                              (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) +
+                               ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z)) * (scale * inv_c2);
             J.last_dphi() = p.g.phi - b.g.phi;   // laplacian of the record, divided there
             J.last_dl() = dl;
         }
