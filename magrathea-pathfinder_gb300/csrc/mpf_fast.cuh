@@ -19,6 +19,7 @@
 //    divisions), TSC weights and field accumulation are FP32, the cosmology
 //    search uses a uniform index table.
 #pragma once
+#include "mpf_fp64.cuh"
 #include "mpf_propagate.cuh"
 
 namespace mpf {
@@ -951,6 +952,12 @@ static __device__ __noinline__ void write_surface(double* o, bool wide_record, d
     }
 }
 
+// v.k / (c k0), the Doppler term of a point
+static __device__ __noinline__ double doppler_of(float v0, float v1, float v2, double k0, double k1, double k2, double k3)
+{
+    return ((double)v0 * k1 + (double)v1 * k2 + (double)v2 * k3) / (kC * k0);
+}
+
 static __device__ __noinline__ double distance_of(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
 
 // a trajectory point's state and the field there
@@ -984,6 +991,14 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // field in the stages and after each step, the octree's levels for the
     // step length, its field for the Jacobian
     constexpr bool born = BORN;
+    // Where the FP64 pipe is the larger part of a step, FP64 operations are
+    // traded for FP32 and integer ones below (a screen of the redshift tests,
+    // the Doppler term formed where it is read, the ISW sum by points, compares
+    // on integer bits): 4 096 CIC rays 3.28 -> 3.09 ms, 8 009 rays with a
+    // velocity field 3.53 -> 3.35.  A plain TSC step with the Jacobian's six
+    // gathers (2 200 instructions) waits for instructions as much as for that
+    // pipe, and the added code made it slower (60 000 map rays 119 -> 126 ms).
+    constexpr bool kLean = ORDER == 1 || VEL;
     Field7 hom;
     clear(hom);
     hom.a = 1.f;
@@ -1012,7 +1027,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         b.k1 *= norm; b.k2 *= norm; b.k3 *= norm;
     }
     const double v0n = VEL ? (P.vobs[0] * b.k1 + P.vobs[1] * b.k2 + P.vobs[2] * b.k3) / (kC * b.k0) : 0.0;
-    double bdop = 0.0;
+    float bv0 = 0.f, bv1 = 0.f, bv2 = 0.f;   // VEL: the velocity at b
     // data != empty (integrator.h:715): with VEL the velocity slots count too
     auto empty = [&](const Field7& f) -> bool { return is_empty(f) && (!VEL || (vv[0] == 0.f && vv[1] == 0.f && vv[2] == 0.f)); };
     b.a = interp_fast(C, b.t, C.a, C.slope_a);
@@ -1038,6 +1053,14 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // instead, which needs no division.  The starting point's redshift is 0.
     const double opc = 1.0 + phi0c2;
     const double inv_c2 = 1.0 / c2;
+    const float inv_c2f = (float)inv_c2;
+    const float opcf = (float)(VEL ? opc - v0n : opc);
+    double x_before = 0.0, y_before = 0.0, z_before = 0.0;
+    float phi_start = 0.f;
+    if (kLean) {
+        phi_start = b.g.phi;
+        x_before = b.x; y_before = b.y; z_before = b.z;
+    }
     // VEL: a0 / a (1 + phi0/c^2 - phi/c^2 + isw + v.k / (c k0) - v0n) - 1
     auto zbracket = [&](float phi, double isw, double dop) -> double {
         if (VEL) return opc - (double)phi * inv_c2 + isw + dop - v0n;
@@ -1051,12 +1074,34 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // the stop at a radius, trajectories), else formed where a record does: its
     // square root is a tenth of the FP64 operations of a CIC step
     const bool want_chi = P.jacobian || skind == STOP_R || (WIDE && O.traj);
+    // FP32 screen of red_above: true only where the point is surely not above.
+    // z1: (1 + zref) / a0 in FP32; the rounding of all terms is below 1e-6 of
+    // the sum of their magnitudes, a tenth of the margin, and a NaN or an
+    // overflow falls through to the float64 test.  A step changes (1 + z) a by
+    // 1e-4 and more, so nearly every step's tests end here: 6 to 12 operations
+    // of the FP64 pipe a test, and with a velocity field the Doppler term's 17.
+    auto red_below = [&](float af, float phi, float iswf, float dopf, float dopm, float z1) -> bool {
+        const float ph = phi * inv_c2f, o = opcf, r = z1 * af;
+        float l = o - ph, m = fabsf(o) + fabsf(ph) + fabsf(r);
+        if (VEL) {
+            l += iswf + dopf;
+            m += fabsf(iswf) + dopm;
+        }
+        return fmaf(1e-5f, m, l) < r;
+    };
+    auto z1_of = [&](double zref) -> float { return (a0 > 0.0) ? (float)((1.0 + zref) / a0) : __int_as_float(0x7fffffff); };
+    auto b_dop = [&]() -> double { return (VEL && k) ? doppler_of(bv0, bv1, bv2, b.k0, b.k1, b.k2, b.k3) : 0.0; };
     // the point b as the reference's photon record
     auto full_point = [&]() -> FastRec {
         FastRec r;
         r.a = b.a; r.t = b.t; r.x = b.x; r.y = b.y; r.z = b.z; r.k0 = b.k0; r.k1 = b.k1; r.k2 = b.k2; r.k3 = b.k3;
-        r.phi = b.g.phi; r.chi = (want_chi || k == 0) ? b.chi : distance_of(b.x, b.y, b.z); r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw(); r.iswold = J.iswold();
-        r.red = (k == 0) ? 0.0 : red_of(b.a, b.g.phi, r.isw, bdop);
+        r.phi = b.g.phi; r.chi = (want_chi || k == 0) ? b.chi : distance_of(b.x, b.y, b.z); r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw();
+        r.iswold = J.iswold();
+        if (kLean && O.final_rec)
+            r.iswold = (J.iswold() + (double)b.g.dx * (b.x - x_before) + (double)b.g.dy * (b.y - y_before) +
+                        (double)b.g.dz * (b.z - z_before)) * (scale * inv_c2) -
+                       ((double)b.g.phi - (double)phi_start) * (2.0 * inv_c2);
+        r.red = (k == 0) ? 0.0 : red_of(b.a, b.g.phi, r.isw, b_dop());
         r.rho = b.g.rho; r.dx = b.g.dx; r.dy = b.g.dy; r.dz = b.g.dz; r.dt = bdt; r.ah = bah;
         r.level = (here.cell >= 0) ? here.level : 0;
         return r;
@@ -1085,8 +1130,9 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         ++next_plane;
     }
     const float two_c2 = (float)(2.0 / c2);
-    const float inv_c2f = (float)(1.0 / c2);
     bool go = !empty(b.g);
+    const float z_stop = (kLean && skind == STOP_REDSHIFT) ? z1_of(stop_ref) : 0.f;
+    float z_next = (kLean && skind == STOP_REDSHIFT && next_plane < np) ? z1_of(SRC ? stop_ref : rpl[next_plane]) : 0.f;
     while (go) {
         if (k >= P.max_steps) { status |= 1u; break; }
         // ---- RK4 step (integrator.h:718-734).  The state stays FP64 and is
@@ -1116,8 +1162,9 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         float tnext;
         {
             const int n = C.n;
-            while (tb < n && !(b.t < __ldg(C.t + tb))) ++tb;
-            while (tb > 0 && b.t < __ldg(C.t + tb - 1)) --tb;
+            auto before = [](double a, double c) -> bool { return kLean ? less64(a, c) : a < c; };
+            while (tb < n && !before(b.t, __ldg(C.t + tb))) ++tb;
+            while (tb > 0 && before(b.t, __ldg(C.t + tb - 1))) --tb;
             ib = tb + (n > 1) * ((tb <= 0) - (tb >= n));
             if (n > 1) {
                 adb = __ldg(C.dadt + ib - 1) + __ldg(C.slope_dadt + ib - 1) * (b.t - __ldg(C.t + ib - 1));
@@ -1273,13 +1320,15 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
             const uint32_t last = (q.cell >= 0) ? (uint32_t)((1ull << q.level) - 1ull) : 0u;
             const bool face = (q.cell < 0) || q.c[0] == 0u || q.c[1] == 0u || q.c[2] == 0u ||
                               q.c[0] >= last || q.c[1] >= last || q.c[2] >= last;
-            if (p.a < 0.0 || (face && !((p.x > mn) && (p.x < mx) && (p.y > mn) && (p.y < mx) && (p.z > mn) && (p.z < mx)))) {
+            if ((kLean ? negative(p.a) : p.a < 0.0) ||
+                (face && !((p.x > mn) && (p.x < mx) && (p.y > mn) && (p.y < mx) && (p.z > mn) && (p.z < mx)))) {
                 clear(p.g);
                 if (VEL) vv[0] = vv[1] = vv[2] = 0.f;
             }
         }
         if (empty(p.g)) break;   // the new point is not appended: the ray ends at b
-        const double pdop = VEL ? ((double)vv[0] * p.k1 + (double)vv[1] * p.k2 + (double)vv[2] * p.k3) / (kC * p.k0) : 0.0;
+        // formed where a redshift is
+        auto p_dop = [&]() -> double { return VEL ? doppler_of(vv[0], vv[1], vv[2], p.k0, p.k1, p.k2, p.k3) : 0.0; };
         const float pdt = -p.g.dt;
         const double b_isw = J.isw(), b_s = J.s(), b_lambda = J.lambda();
         const double p_isw = b_isw + (double)((bdt + pdt) * dtf * inv_c2f);
@@ -1289,16 +1338,31 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         J.s() = p_s;
         J.lambda() = p_lambda;
         if (O.final_rec || (WIDE && traj)) {   // reported by photon records only
-            if (O.final_rec)
+            // the sum of (g_b + g_p).(x_p - x_b) over the steps, gathered by
+            // point: g_k.(x_k+1 - x_k-1), the last point's part where it is read
+            if (kLean && O.final_rec) {
+                J.iswold() += (double)b.g.dx * (p.x - x_before) + (double)b.g.dy * (p.y - y_before) + (double)b.g.dz * (p.z - z_before);
+                x_before = b.x; y_before = b.y; z_before = b.z;
+            } else if (O.final_rec) {
                 J.iswold() -= ((double)p.g.phi - (double)b.g.phi) * (2.0 * inv_c2) -
                               (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) +
                                ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z)) * (scale * inv_c2);
+            }
             J.last_dphi() = p.g.phi - b.g.phi;   // laplacian of the record, divided there
             J.last_dl() = dl;
         }
         if (want_chi) p.chi = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
         dl = (q.cell >= 0 ? cell_extent(q.level) : 0.0) * (p.a * p.a * ratio_k);
         ++k;
+        const float paf = kLean ? (float)p.a : 0.f;
+        float iswf = 0.f, dopf = 0.f, dopm = 0.f;   // dopm: the sum of its terms' magnitudes
+        if (VEL && skind == STOP_REDSHIFT) {
+            iswf = (float)p_isw;
+            const float w = 1.f / ((float)kC * (float)p.k0);
+            const float d1v = vv[0] * (float)p.k1 * w, d2v = vv[1] * (float)p.k2 * w, d3v = vv[2] * (float)p.k3 * w;
+            dopf = d1v + d2v + d3v;
+            dopm = fabsf(d1v) + fabsf(d2v) + fabsf(d3v);
+        }
         // the surfaces the step crossed: everything but the Jacobian, from b and p
         const int first_crossed = next_plane;
         bool p_red_known = false;   // the stop test below reads p's redshift where a surface formed it
@@ -1309,9 +1373,9 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
             bool crossed;
             double q1 = 0.0;
             if (!kj && skind == STOP_REDSHIFT) {
-                crossed = red_above(p.a, p.g.phi, p_isw, pdop, ref);
+                crossed = !(kLean && red_below(paf, p.g.phi, iswf, dopf, dopm, z_next)) && red_above(p.a, p.g.phi, p_isw, p_dop(), ref);
             } else {
-                if (!kj && skind == STOP_PLANE && !p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, pdop); p_red_known = true; }
+                if (!kj && skind == STOP_PLANE && !p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, p_dop()); p_red_known = true; }
                 q1 = kj ? (p.x * kj[0] + p.y * kj[1] + p.z * kj[2])
                    : (skind == STOP_R) ? p.chi : (skind == STOP_LAMBDA) ? p_lambda : (skind == STOP_T) ? p.t
                    : (skind == STOP_A) ? p.a : (skind == STOP_S) ? p_s : p_red;
@@ -1319,10 +1383,11 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
             }
             if (!crossed) break;
             const int j = next_plane++;
+            if (kLean && !SRC && skind == STOP_REDSHIFT && next_plane < np) z_next = z1_of(rpl[next_plane]);
             cross_k[j] = k;
             if (prow) {
-                if (!p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, pdop); p_red_known = true; }
-                const double b_red = (k == 1) ? 0.0 : red_of(b.a, b.g.phi, b_isw, bdop);
+                if (!p_red_known) { p_red = red_of(p.a, p.g.phi, p_isw, p_dop()); p_red_known = true; }
+                const double b_red = (k == 1) ? 0.0 : red_of(b.a, b.g.phi, b_isw, b_dop());
                 const double b_chi = want_chi ? b.chi : (k == 1) ? 0.0 : distance_of(b.x, b.y, b.z);
                 const double p_chi = want_chi ? p.chi : distance_of(p.x, p.y, p.z);
                 double* o = prow + j * rec_fields;
@@ -1345,7 +1410,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         b = p;
         bdt = pdt;
         bah = p.g.a;
-        bdop = pdop;
+        if (VEL) { bv0 = vv[0]; bv1 = vv[1]; bv2 = vv[2]; }
         if (kind != kSpotSame) {
             if (kind == kSpotLeaf) {
                 // +-w or 0 per axis (selects, no int-to-double conversion)
@@ -1417,7 +1482,11 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         switch (skind) {
         case STOP_R: stop = b.chi > stop_ref; break;
         case STOP_LAMBDA: stop = J.lambda() > stop_ref; break;
-        case STOP_REDSHIFT: stop = p_red_known ? (p_red > stop_ref) : red_above(b.a, b.g.phi, J.isw(), bdop, stop_ref); break;
+        case STOP_REDSHIFT:
+            stop = p_red_known ? (p_red > stop_ref)
+                               : !(kLean && red_below(paf, b.g.phi, iswf, dopf, dopm, z_stop)) &&
+                                     red_above(b.a, b.g.phi, J.isw(), b_dop(), stop_ref);
+            break;
         case STOP_T: stop = b.t > stop_ref; break;
         case STOP_A: stop = b.a < stop_ref; break;
         case STOP_PLANE: {

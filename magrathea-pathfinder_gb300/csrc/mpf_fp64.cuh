@@ -4,9 +4,10 @@
 // pipes take 1 to 2); the functions below give the bits of the hardware's
 // conversions, products with powers of two and compares in 4 to 10 integer
 // instructions, and leave zeros, subnormals, infinities and NaN to it.  They
-// pay where that pipe is the bound (the float64 kernel, the deposit), not in
-// the FP32-gather kernel, whose conversions overlap its other latencies
-// (there they measured 3 to 10 % slower).
+// pay where that pipe is the bound: the float64 kernel, the deposit, the
+// compares of the FP32-gather kernel's CIC and velocity instantiations.  That
+// kernel's conversions overlap its other latencies (on integer bits they
+// measured 3 to 10 % slower).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -54,5 +55,8 @@ __device__ __forceinline__ bool less64(double a, double b)
     y ^= (long long)((unsigned long long)(y >> 63) >> 1);
     return x < y;
 }
+
+// a < 0 (a NaN with its sign set reads as negative)
+__device__ __forceinline__ bool negative(double a) { return (unsigned long long)__double_as_longlong(a) > 0x8000000000000000ull; }
 
 }  // namespace mpf

@@ -193,3 +193,25 @@ def test_deposit_matches_oracle_at_tile_edges(gpu_lib, pkg, oracle_mod, synth, a
     ov, orho = O.deposit_velocity(pos, pv, scheme)
     np.testing.assert_array_equal(rho.view(np.uint32), np.asarray(orho, dtype=np.float32).view(np.uint32))
     np.testing.assert_array_equal(v.view(np.uint32), np.asarray(ov, dtype=np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("velocity", [True, False])
+def test_redshift_tests_at_the_threshold(gpu_lib, pkg, synth, amr, vel, cosmo, order, velocity):
+    """A ray stopped just below and just above a redshift that it reaches: the
+    tests' FP32 screen must leave both to the float64 comparison.  1e-10 is
+    above the rounding of the redshift and far below the screen's margin."""
+    tree = pkg.Octree.from_records(amr["records"])
+    if velocity:
+        tree.set_velocity(vel["ref_vel_tsc"], vel["ref_rho_tsc"])
+    kw = dict(nsteps=4, order=order, stop="redshift", jacobian=False, vobs=vel["vobs"] if velocity else (0.0, 0.0, 0.0))
+    launch, length = synth.photon_grid(4, 2.0, 2.0), float(amr["cosmo_length"])
+    s0, f0, _, _ = pkg.propagate(tree, cosmo, launch, length, planes=np.array([0.02]), **kw)
+    red = f0[:, pkg.PHOTON_FIELDS.index("redshift")]
+    for i in range(0, launch.shape[0], 3):
+        for shift, more in ((-1e-10, 0), (1e-10, 1)):
+            z = red[i] * (1.0 + shift)
+            s, f, p, rc = pkg.propagate(tree, cosmo, launch[i:i + 1], length, planes=np.array([z]), **kw)
+            assert rc == 0 and s[0] == s0[i] + more, (i, shift)
+            assert p[0, 0, 0] == s[0] - 2, (i, shift)
+    tree.close()
