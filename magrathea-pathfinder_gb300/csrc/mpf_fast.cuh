@@ -927,8 +927,8 @@ __device__ __forceinline__ void jac_fast(const DevTree& T, const Spot& here, dou
 struct SurfaceEnd {
     double x, y, z, t, a, red, chi, lambda, s, isw, rho, phi, k0, k1, k2, k3;
 };
-static __device__ __noinline__ void write_surface(double* o, bool wide_record, double first, double f, SurfaceEnd b, SurfaceEnd p,
-                                                  double rmax)
+__device__ __forceinline__ void surface_record(double* o, bool wide_record, double first, double f, const SurfaceEnd& b,
+                                               const SurfaceEnd& p, double rmax)
 {
     const double px = b.x * f + p.x * (1 - f), py = b.y * f + p.y * (1 - f), pz = b.z * f + p.z * (1 - f);
     o[0] = first; o[1] = f; o[2] = px; o[3] = py; o[4] = pz; o[5] = sqrt(px * px + py * py + pz * pz);
@@ -950,6 +950,12 @@ static __device__ __noinline__ void write_surface(double* o, bool wide_record, d
         o[22] = b.k2 * f + p.k2 * (1 - f);
         o[23] = b.k3 * f + p.k3 * (1 - f);
     }
+}
+
+static __device__ __noinline__ void write_surface(double* o, bool wide_record, double first, double f, SurfaceEnd b, SurfaceEnd p,
+                                                  double rmax)
+{
+    surface_record(o, wide_record, first, f, b, p, rmax);
 }
 
 // v.k / (c k0), the Doppler term of a point
@@ -999,6 +1005,12 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // gathers (2 200 instructions) waits for instructions as much as for that
     // pipe, and the added code made it slower (60 000 map rays 119 -> 126 ms).
     constexpr bool kLean = ORDER == 1 || VEL;
+    // Stage 1 written out, the table slope kept for the step and the surface
+    // record out of line pay everywhere but in the TSC source instantiation,
+    // which the catalogue's persistent kernel inlines: there they cost 5 to 8 %
+    // (16 384 sources on an AMR octree 236 -> 225 ms without them, 2 054 on a
+    // uniform one 20.1 -> 18.7).
+    constexpr bool kPlain = SRC && ORDER == 2;
     Field7 hom;
     clear(hom);
     hom.a = 1.f;
@@ -1174,14 +1186,14 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
                 tnext = __int_as_float(0x7f800000);
             }
         }
-        const float seg0 = (C.n > 1) ? __ldg(&C.seg[ib - 1].x) : 0.f;
+        const float seg0 = (!kPlain && C.n > 1) ? __ldg(&C.seg[ib - 1].x) : 0.f;
         // da/dt(b.t + dt) - da/dt(b.t) along the table's pieces (dt >= 0; the
         // last piece extends past the table's end, as in Utility::interpolate)
         auto dadot = [&](float dt) -> float {
             if (C.n <= 1) return 0.f;
-            if (!(dt > tnext)) return seg0 * dt;
+            if (!kPlain && !(dt > tnext)) return seg0 * dt;
             float tn = tnext, rem = dt, r = 0.f;
-            float sl = seg0;
+            float sl = kPlain ? __ldg(&C.seg[ib - 1].x) : seg0;
             int j = ib;
             for (int guard = 0; rem > tn && guard < 64; ++guard) {
                 r = fmaf(sl, tn, r);
@@ -1218,7 +1230,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         // increments (written out: 3 to 7 % of a step of 2200 instructions);
         // stages 2-4 are located from their FP32 offset to b's cell, the
         // post-step point from its float64 offset
-        {
+        if (!kPlain) {
             // stage 1, at b: no increments, the drag of b itself
             const float gk = fmaf(g.dx, kb1, fmaf(g.dz, kb3, __fmul_rn(g.dy, kb2)));
             const float dphidl = fmaf(g.dt, kb0, gk);
@@ -1234,10 +1246,10 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
             d1 = fmaf(coef, kb1, -G1); d2 = fmaf(coef, kb2, -G2); d3 = fmaf(coef, kb3, -G3);
             dA = kb0 * adbf;
         }
-        // stages 2-4
+        // stages 2-4 (rolled: 1-4)
 #pragma unroll 1
-        for (int sg = 1; sg < 5; ++sg) {
-            const float cfr = (sg < 3) ? 0.5f : 1.f;
+        for (int sg = kPlain ? 0 : 1; sg < 5; ++sg) {
+            const float cfr = (kPlain && sg == 0) ? 0.f : (sg < 3) ? 0.5f : 1.f;
             if (sg == 4) {
                 const double dl6 = dl * (1.0 / 6.0), dlL6 = dlL * (1.0 / 6.0);
                 const float dl6f = (float)dl6, dlL6f = (float)dlL6;
@@ -1259,7 +1271,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
                 ds = sqrtf(ex * ex + ey * ey + ez * ez);
                 dtf = fmaf(dlf, kb0, dl6f * S0);
             }
-            if (!born || sg == 4) {
+            if ((!kPlain || sg > 0) && (!born || sg == 4)) {
                 float rx, ry, rz;
                 if (sg == 4) {
                     rx = (float)(p.x - J.cen(0)) * cpu; ry = (float)(p.y - J.cen(1)) * cpu; rz = (float)(p.z - J.cen(2)) * cpu;
@@ -1276,10 +1288,10 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
                 if (!born) g = gather_spot<ORDER, VEL>(T, q, r7, ps, sg == 4, vv);
             }
             if (sg < 4) {
-                if (born) g = hom;
+                if (born && (!kPlain || sg > 0)) g = hom;
                 const float cdl = cfr * dlf;
                 const float q0 = __fmul_rn(cdl, d0), q1 = __fmul_rn(cdl, d1), q2 = __fmul_rn(cdl, d2), q3 = __fmul_rn(cdl, d3);
-                const float w = (sg == 3) ? 1.f : 2.f;
+                const float w = ((kPlain && sg == 0) || sg == 3) ? 1.f : 2.f;
                 const float k0 = kb0 + q0, k1 = kb1 + q1, k2 = kb2 + q2, k3 = kb3 + q3;
                 const float as = fmaf(cdl, dA, abf);
                 const float dad = dadot(cdl * pk0);
@@ -1399,7 +1411,8 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
                                     b.k0, b.k1, b.k2, b.k3};
                 const SurfaceEnd e1{p.x, p.y, p.z, p.t, p.a, p_red, p_chi, p_lambda, p_s, p_isw, (double)p.g.rho, (double)p.g.phi,
                                     p.k0, p.k1, p.k2, p.k3};
-                write_surface(o, SRC || WIDE, (double)(k - 1), (q1 - ref) / (q1 - q0), e0, e1, (k >= 2) ? (double)J.rmax() : 0.0);
+                if (kPlain) surface_record(o, SRC || WIDE, (double)(k - 1), (q1 - ref) / (q1 - q0), e0, e1, (k >= 2) ? (double)J.rmax() : 0.0);
+                else write_surface(o, SRC || WIDE, (double)(k - 1), (q1 - ref) / (q1 - q0), e0, e1, (k >= 2) ? (double)J.rmax() : 0.0);
             }
         }
         // the largest density of the points before the new one
