@@ -54,16 +54,16 @@ UNIT = "photon-steps/s"
 # + post-step 27 x 28 B + Jacobian 6 x 27 x 12 B
 BYTES_PER_PHOTON_STEP = 4 * 27 * 16 + 27 * 28 + 6 * 27 * 12
 # DRAM bytes per photon-step of the propagate kernel, from one ncu capture of the
-# same kernel on the medium octree (65 536 rays to z = 0.5): (37.66 + 1.93) MB
+# same kernel on the medium octree (65 536 rays to z = 0.5): (37.25 + 1.58) MB
 # over 6.95e7 photon-steps; the bench's per-launch traffic is this figure times
 # the photon-steps of a launch
-DRAM_BYTES_PER_PHOTON_STEP = 0.57
+DRAM_BYTES_PER_PHOTON_STEP = 0.56
 # FP64 add + fma + mul thread operations per photon-step of the same capture
 # (smsp__sass_thread_inst_executed_op_{dadd,dfma,dmul}_pred_on): the
 # arithmetic that bounds the kernel on this part, whose FP64 pipe retires 2
 # operations per SM per cycle (sm__sass_thread_inst_executed_op_dfma_pred_on
 # .sum.peak_sustained = 304 per cycle for 152 SMs)
-FP64_OPS_PER_PHOTON_STEP = 137
+FP64_OPS_PER_PHOTON_STEP = 80
 FP64_OPS_PER_SM_CYCLE = 2
 
 
