@@ -1086,6 +1086,9 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // the stop at a radius, trajectories), else formed where a record does: its
     // square root is a tenth of the FP64 operations of a CIC step
     const bool want_chi = P.jacobian || skind == STOP_R || (WIDE && O.traj);
+    // the running ISW column: read by photon records only, the final one's and
+    // a trajectory's
+    const bool want_iswold = O.final_rec || (WIDE && O.traj);
     // FP32 screen of red_above: true only where the point is surely not above.
     // z1: (1 + zref) / a0 in FP32; the rounding of all terms is below 1e-6 of
     // the sum of their magnitudes, a tenth of the margin, and a NaN or an
@@ -1109,7 +1112,7 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         r.a = b.a; r.t = b.t; r.x = b.x; r.y = b.y; r.z = b.z; r.k0 = b.k0; r.k1 = b.k1; r.k2 = b.k2; r.k3 = b.k3;
         r.phi = b.g.phi; r.chi = (want_chi || k == 0) ? b.chi : distance_of(b.x, b.y, b.z); r.lambda = J.lambda(); r.s = J.s(); r.isw = J.isw();
         r.iswold = J.iswold();
-        if (kLean && O.final_rec)
+        if (kLean && want_iswold)
             r.iswold = (J.iswold() + (double)b.g.dx * (b.x - x_before) + (double)b.g.dy * (b.y - y_before) +
                         (double)b.g.dz * (b.z - z_before)) * (scale * inv_c2) -
                        ((double)b.g.phi - (double)phi_start) * (2.0 * inv_c2);
@@ -1349,13 +1352,13 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
         J.isw() = p_isw;
         J.s() = p_s;
         J.lambda() = p_lambda;
-        if (O.final_rec || (WIDE && traj)) {   // reported by photon records only
+        if (want_iswold) {
             // the sum of (g_b + g_p).(x_p - x_b) over the steps, gathered by
             // point: g_k.(x_k+1 - x_k-1), the last point's part where it is read
-            if (kLean && O.final_rec) {
+            if (kLean) {
                 J.iswold() += (double)b.g.dx * (p.x - x_before) + (double)b.g.dy * (p.y - y_before) + (double)b.g.dz * (p.z - z_before);
                 x_before = b.x; y_before = b.y; z_before = b.z;
-            } else if (O.final_rec) {
+            } else {
                 J.iswold() -= ((double)p.g.phi - (double)b.g.phi) * (2.0 * inv_c2) -
                               (((double)b.g.dx + (double)p.g.dx) * (p.x - b.x) + ((double)b.g.dy + (double)p.g.dy) * (p.y - b.y) +
                                ((double)b.g.dz + (double)p.g.dz) * (p.z - b.z)) * (scale * inv_c2);

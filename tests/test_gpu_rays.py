@@ -59,6 +59,37 @@ def test_bundles_fast_within_tolerance(rays_dev, pkg, order):
         assert np.all(np.abs(got[:, 22] - want[:, 22]) <= 1e-5 * np.abs(want[:, 22]) + 1e-30)
 
 
+@pytest.mark.parametrize("order", [1, 2])
+def test_bundles_fast_records_every_column(rays_dev, pkg, order):
+    """Every directly stored column of a fast trajectory against the exact
+    mode's.  A fast gather is good to 2e-6 of the field's scale and the state to
+    better, so a column agrees to 1e-5 of its largest value, and the two running
+    sums to 1e-5 of the sum of their terms at the field's largest values: isw of
+    2 |dphidt| dt / c^2, iswold of (2 |grad phi| dx length + 2 |phi|) / c^2.  A
+    sum that the exact mode reports is never all zero."""
+    g, tree, cos = rays_dev
+    c2 = 299792458.0 ** 2
+    length = float(g["cosmo_length"])
+    seen = 0
+    for i in range(g["ref_sizes_o%d" % order].shape[0]):
+        se, te = _run(pkg, g, tree, cos, i, order, True)
+        sf, tf = _run(pkg, g, tree, cos, i, order, False)
+        m = int(min(se[0], sf[0])) - 1
+        if m < 2:
+            continue
+        e, f = te[0, :m], tf[0, :m]
+        for col in (1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 19, 22, 25, 26, 27, 28):
+            assert np.abs(f[:, col] - e[:, col]).max() <= 1e-5 * np.abs(e[:, col]).max() + 1e-30, (i, col)
+        units = {23: 2 * np.abs(e[:, 27]).max() * np.abs(np.diff(e[:, 2])).sum() / c2,
+                 24: (2 * np.abs(e[:, 14:17]).max() * np.abs(np.diff(e[:, 3:6], axis=0)).sum() * length +
+                      2 * np.abs(e[:, 13]).max()) / c2}
+        for col, unit in units.items():
+            assert np.abs(f[:, col] - e[:, col]).max() <= 1e-5 * unit, (i, col)
+            assert f[:, col].any() == e[:, col].any(), (i, col)
+            seen += int(e[:, col].any())
+    assert seen
+
+
 def test_batch_of_bundles_matches_oracle(rays_dev, pkg, oracle_mod, synth):
     """Many bundles in one call (the trajectory buffers hold all of them at
     once) against the C oracle, exact mode."""
