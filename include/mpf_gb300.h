@@ -190,7 +190,11 @@ int mpf_propagate_accuracy(const mpf_octree* o, const mpf_cosmology* c, const mp
 
 /* Same with device buffers, asynchronous on `stream` (a cudaStream_t, or NULL
  * for the legacy default stream).  status_device: one uint32 in device memory
- * that receives warning bits (bit 0: max_steps reached). */
+ * that receives warning bits (bit 0: max_steps reached).  A batch of 2^14 to
+ * 2^22 rays on a refined octree is traced in the order of its directions: the
+ * order lies in one of at most eight 16 MiB buffers, made by the octree's first
+ * such calls (cudaMalloc) and freed with it; a call under stream capture, or
+ * one that finds every buffer at work on other streams, keeps the given order. */
 int mpf_propagate_device(const mpf_octree* o, const mpf_cosmology* c, const mpf_params* p, int64_t n,
                          const double* launch_device, int64_t* steps_device, double* final_device,
                          double* plane_device, uint32_t* status_device, void* stream);

@@ -216,32 +216,119 @@ static __global__ void k_order_scatter(const double* __restrict__ launch, long l
     if (i < n) perm[atomicAdd(w + order_bin(launch + 6 * i, w + kOrderBins), 1u)] = (int)i;
 }
 
-// Memory of the orders, per device, octree and stream (per thread too where
-// one stream handle stands for a stream of each thread), as the calls on one
-// stream are ordered: at most 16 MiB each, freed with the octree.
-using OrderKey = std::tuple<int, const void*, cudaStream_t, std::thread::id>;
-struct OrderMemory {
+// Memory of the orders: at most kOrderBuffers buffers per device and octree,
+// each of the largest batch's size (16 MiB, so that none is ever replaced or
+// outgrown), made when a call finds none free and freed with the octree.  A
+// call claims one until its last kernel is queued and records the buffer's
+// event behind that.  A buffer is free again once its event has passed, or for
+// the stream whose work it still serves; whoever takes it waits for the event
+// on its own stream, so that a stream handle or thread that comes again cannot
+// read or write it early.  With none free (more calls in flight on different
+// streams than buffers) a call traces in the caller's order.
+constexpr int kOrderBuffers = 8;
+struct OrderBuffer {
     unsigned* p = nullptr;
-    long long rays = 0;
+    cudaEvent_t done = nullptr;
+    cudaStream_t stream = nullptr;   // of the last call (and its thread, where a handle stands for a stream of each)
+    std::thread::id who;
+    bool claimed = false;
+};
+struct OrderPool {
+    OrderBuffer buffer[kOrderBuffers];
 };
 static std::mutex g_order_mu;
-static std::map<OrderKey, OrderMemory> g_orders;
+static std::map<std::pair<int, const void*>, OrderPool> g_orders;
+
+// A capture of another thread must not see this thread's allocation or event
+// queries as its own.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 static void free_orders(const void* keys)
 {
     std::lock_guard<std::mutex> lock(g_order_mu);
     for (auto it = g_orders.begin(); it != g_orders.end();) {
-        if (std::get<1>(it->first) == keys) {
-            cudaFree(it->second.p);
-            it = g_orders.erase(it);
-        } else {
+        if (it->first.second != keys) {
             ++it;
+            continue;
         }
+        for (OrderBuffer& b : it->second.buffer) {
+            if (b.p) cudaFree(b.p);
+            if (b.done) cudaEventDestroy(b.done);
+        }
+        it = g_orders.erase(it);
     }
 }
 
-// The order of a batch's rays on the device, or null where the caller's stays.
-static cudaError_t order_rays(const DevTree& T, const double* d_launch, long long n, int sms, cudaStream_t s, const int** perm)
+// A call's hold on a buffer, given back behind the work queued on its stream.
+struct OrderClaim {
+    OrderBuffer* b = nullptr;
+    cudaStream_t stream = nullptr;
+    std::thread::id who;
+    OrderClaim() = default;
+    OrderClaim(const OrderClaim&) = delete;
+    OrderClaim& operator=(const OrderClaim&) = delete;
+    ~OrderClaim()
+    {
+        if (!b) return;
+        const bool queued = !b->p || cudaEventRecord(b->done, stream) == cudaSuccess;
+        std::lock_guard<std::mutex> lock(g_order_mu);
+        b->stream = stream;
+        b->who = who;
+        b->claimed = !queued;   // without its event nobody may take it again
+    }
+    // a buffer for work on s; false: none is free, or there is no memory
+    bool take(int dev, const void* keys, cudaStream_t s)
+    {
+        const OutsideCapture outside;
+        const std::thread::id id = (s == cudaStreamPerThread) ? std::this_thread::get_id() : std::thread::id();
+        OrderBuffer* got = nullptr;
+        {
+            std::lock_guard<std::mutex> lock(g_order_mu);
+            OrderBuffer *own = nullptr, *idle = nullptr, *fresh = nullptr;
+            for (OrderBuffer& q : g_orders[std::make_pair(dev, keys)].buffer) {
+                if (q.claimed) continue;
+                if (!q.p) {
+                    if (!fresh) fresh = &q;
+                } else if (q.stream == s && q.who == id) {
+                    own = &q;
+                } else if (!idle) {
+                    if (cudaEventQuery(q.done) == cudaSuccess) idle = &q;
+                    else (void)cudaGetLastError();   // not ready
+                }
+            }
+            got = own ? own : idle ? idle : fresh;
+            if (!got) return false;
+            got->claimed = true;
+        }
+        b = got;
+        stream = s;
+        who = id;
+        if (b->p) return cudaStreamWaitEvent(s, b->done, 0) == cudaSuccess;
+        if (cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess) {
+            (void)cudaGetLastError();
+            b->done = nullptr;
+            return false;
+        }
+        if (cudaMalloc(&b->p, (size_t)(kOrderBins + 4 + kOrderMaxRays) * sizeof(int)) != cudaSuccess) {
+            (void)cudaGetLastError();   // no room
+            b->p = nullptr;
+            cudaEventDestroy(b->done);
+            b->done = nullptr;
+            return false;
+        }
+        return true;
+    }
+};
+
+// The order of a batch's rays on the device, in the buffer of `claim` (to be
+// held until the last kernel that reads it is queued), or null where the
+// caller's stays.
+static cudaError_t order_rays(const DevTree& T, const double* d_launch, long long n, int sms, cudaStream_t s, OrderClaim& claim,
+                              const int** perm)
 {
     *perm = nullptr;
     if (n < kOrderMinRays || n > kOrderMaxRays || T.Lmax <= T.Lt) return cudaSuccess;
@@ -254,24 +341,8 @@ static cudaError_t order_rays(const DevTree& T, const double* d_launch, long lon
     int dev = 0;
     const cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    unsigned* w = nullptr;
-    {
-        const std::thread::id who = (s == cudaStreamPerThread) ? std::this_thread::get_id() : std::thread::id();
-        std::lock_guard<std::mutex> lock(g_order_mu);
-        OrderMemory& m = g_orders[OrderKey(dev, T.keys, s, who)];
-        if (m.rays < n) {
-            const long long rays = std::min(kOrderMaxRays, std::max(n, 2 * m.rays));
-            cudaFree(m.p);   // waits for the work that reads it
-            m = OrderMemory{};
-            if (cudaMalloc(&m.p, (size_t)(kOrderBins + 4 + rays) * sizeof(int)) != cudaSuccess) {
-                (void)cudaGetLastError();   // no room: the caller's order
-                m = OrderMemory{};
-                return cudaSuccess;
-            }
-            m.rays = rays;
-        }
-        w = m.p;
-    }
+    if (!claim.take(dev, T.keys, s)) return cudaSuccess;
+    unsigned* const w = claim.b->p;
     int* const order = reinterpret_cast<int*>(w + kOrderBins + 4);
     const unsigned blocks = (unsigned)((n + 255) / 256);
     k_order_reset<<<(kOrderBins + 4 + 255) / 256, 256, 0, s>>>(w);
@@ -463,7 +534,8 @@ cudaError_t launch_propagate<false>(const DevTree& T, const DevCosmo& C, const P
     if (e != cudaSuccess) return e;
     FastShape shape = fast_launch_shape(n, st.blocks_per_sm, st.sms, P.jacobian != 0);
     const int* perm = nullptr;
-    if (fast_mode(T, P, O) >= 6 && (e = order_rays(T, d_launch, n, st.sms, stream, &perm)) != cudaSuccess) return e;
+    OrderClaim claim;
+    if (fast_mode(T, P, O) >= 6 && (e = order_rays(T, d_launch, n, st.sms, stream, claim, &perm)) != cudaSuccess) return e;
     int depth = 1;
 #if MPF_DIAG
     // MPF_STATS=1: print the counts of the rare paths (diagnostics; serialises the call)
