@@ -2,6 +2,7 @@
 // records, FP64 RK4 state (with FMA).
 #include "mpf_fast.cuh"
 #include "mpf_internal.h"
+#include "mpf_tune.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -395,7 +396,8 @@ static cudaError_t fast_launch_state(cudaStream_t stream, FastLaunchState* out)
 // Autotuner of the persistent launch shape: threads per block and the depth
 // of a warp's claim on the work queue (32 x depth rays).  The first batch of
 // at least kTuneMinRays rays for a (device, octree, kernel mode) is split into
-// one slice per candidate shape; each slice is traced with its shape and
+// one slice per candidate shape (mpf_tune.h; contiguous parts of the caller's
+// list where the rays are not reordered); each slice is traced with its shape and
 // timed with CUDA events, and its photon-steps are summed on the device.  The
 // shape with the most photon-steps per second is kept for that key and used
 // by every later launch.  Every ray is traced exactly once and its results do
@@ -405,7 +407,7 @@ struct TuneShape {
     int tpb, depth;
 };
 static const TuneShape kTuneCandidates[] = {{kFastThreads, 1}, {64, 1}, {32, 1}, {kFastThreads, 2}};
-constexpr int kTuneN = 4;
+constexpr int kTuneN = kTuneSlices;
 constexpr long long kTuneMinRays = 1ll << 17;
 
 struct TuneResult {
@@ -427,6 +429,12 @@ static __global__ void k_sum_steps(const long long* __restrict__ steps, const in
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
+}
+
+static __global__ void k_deal(const int* __restrict__ perm, long long n, int* __restrict__ dealt)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dealt[i] = perm[tune_dealt(i, n)];
 }
 
 // resident blocks per SM of the kernel at tpb threads (at least 1)
@@ -451,12 +459,19 @@ static cudaError_t tune_and_launch(const DevTree& T, const DevCosmo& C, const Pr
                                    TuneResult* res)
 {
     unsigned long long* dsum = nullptr;
+    int* dealt = nullptr;
     cudaEvent_t ev[kTuneN + 1] = {};
     cudaError_t e = cudaMalloc(&dsum, kTuneN * sizeof(unsigned long long));
+    if (e == cudaSuccess && perm) e = cudaMalloc(&dealt, (size_t)n * sizeof(int));
+    if (e == cudaSuccess && perm) {
+        k_deal<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(perm, n, dealt);
+        perm = dealt;
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(dsum, 0, kTuneN * sizeof(unsigned long long), stream);
     for (int k = 0; k <= kTuneN && e == cudaSuccess; ++k) e = cudaEventCreate(&ev[k]);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], stream);
-    const long long slice = n / kTuneN;
+    const long long slice = perm ? tune_slice(n) : n / kTuneN;
     for (int k = 0; k < kTuneN && e == cudaSuccess; ++k) {
         const long long lo = k * slice, hi = (k == kTuneN - 1) ? n : lo + slice;
         const TuneShape& sh = kTuneCandidates[k];
@@ -486,6 +501,7 @@ static cudaError_t tune_and_launch(const DevTree& T, const DevCosmo& C, const Pr
     }
     for (int k = 0; k <= kTuneN; ++k)
         if (ev[k]) cudaEventDestroy(ev[k]);
+    if (dealt) cudaFree(dealt);   // the slices are done: waited for above, or by this call
     if (dsum) cudaFree(dsum);
     return e;
 }
