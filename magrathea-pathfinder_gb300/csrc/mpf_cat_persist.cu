@@ -258,7 +258,9 @@ __global__ void MPF_FAST_BOUNDS k_cat_persistent(DevTree T, DevCosmo C, CatPlanD
             }
         }
         // the item's state was written by the warp that queued it, on any SM:
-        // nothing of it may come from this SM's L1
+        // nothing of it may come from this SM's L1.  Every lane that reads it
+        // fences after the first lane's poll (__shfl_sync orders no memory)
+        __syncwarp();
         __threadfence();
         item = __shfl_sync(0xffffffffu, item, lane - R.sub);
         if (ray >= cnt) item = -1;

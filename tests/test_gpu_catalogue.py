@@ -222,3 +222,19 @@ def test_catalogue_work_queue_plan_reuse(cat_setup, pkg):
     big, st_big, _ = _run(pkg, g, tree, cos, 2, False, 1e-8, src=np.tile(src, (reps, 1)))
     np.testing.assert_array_equal(big.view(np.uint64), np.tile(ref, (reps, 1)).view(np.uint64))
     assert st_big["rays"] == reps * st["rays"]
+
+
+@pytest.mark.parametrize("n", (1, 3000, 6000, 9500, 20000))
+def test_catalogue_rows_do_not_depend_on_lanes_a_ray(cat_setup, pkg, n):
+    """Up to 5, 10 and 16 sources a warp are traced with 6, 3 and 2 lanes each,
+    and all of a source's lanes read the state its first lane took from the
+    queue: the rows equal those of a call of few sources bit for bit, call after
+    call."""
+    g, tree, cos = cat_setup
+    src = g["cat_src"]
+    ref, _, _ = _run(pkg, g, tree, cos, 2, False, 1e-8)
+    reps = n // src.shape[0] + 1
+    for _ in range(3):
+        rows, _, rc = _run(pkg, g, tree, cos, 2, False, 1e-8, src=np.tile(src, (reps, 1))[:n])
+        assert rc == 0
+        np.testing.assert_array_equal(rows.view(np.uint64), np.tile(ref, (reps, 1))[:n].view(np.uint64))
