@@ -404,12 +404,18 @@ cudaError_t plan_build(CatPlan& pl, const DevTree& T, const DevCosmo& C, PropPar
     if (e != cudaSuccess) return e;
     D.call = pl.d_call;
     P.ray_stop = D.radius;
+    // a build with larger blocks (MPF_FAST_THREADS) passes the 48 KB that need no opt-in
+    constexpr int smem = kFastThreads * kSharedRaySlotBytes;
+    static_assert(smem <= 227 * 1024, "a block's ray slots exceed an SM's shared memory");
+    if (smem > 48 * 1024) {
+        e = cudaFuncSetAttribute((pl.order == 1) ? (const void*)k_cat_persistent<1> : (const void*)k_cat_persistent<2>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
     // persistent grid: every SM's resident blocks of the propagate launch bounds
     int bps = 0, sms = 0;
-    e = (pl.order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<1>, kFastThreads,
-                                                                          kFastThreads * kSharedRaySlotBytes)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<2>, kFastThreads,
-                                                                          kFastThreads * kSharedRaySlotBytes);
+    e = (pl.order == 1) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<1>, kFastThreads, smem)
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cat_persistent<2>, kFastThreads, smem);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl.device);
     if (e != cudaSuccess) return e;
     pl.tpb = kFastThreads;
