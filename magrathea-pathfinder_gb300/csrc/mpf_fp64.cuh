@@ -56,7 +56,10 @@ __device__ __forceinline__ bool less64(double a, double b)
     return x < y;
 }
 
-// a < 0 (a NaN with its sign set reads as negative)
-__device__ __forceinline__ bool negative(double a) { return (unsigned long long)__double_as_longlong(a) > 0x8000000000000000ull; }
+// a < 0: the bits of the negative numbers up to -infinity (neither -0 nor a NaN)
+__device__ __forceinline__ bool negative(double a)
+{
+    return (unsigned long long)__double_as_longlong(a) - 0x8000000000000001ull < 0x7ff0000000000000ull;
+}
 
 }  // namespace mpf
