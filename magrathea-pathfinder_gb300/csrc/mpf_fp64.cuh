@@ -12,6 +12,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "mpf_keys.cuh"
+
 namespace mpf {
 
 // (double)v
@@ -60,6 +62,39 @@ __device__ __forceinline__ bool less64(double a, double b)
 __device__ __forceinline__ bool negative(double a)
 {
     return (unsigned long long)__double_as_longlong(a) - 0x8000000000000001ull < 0x7ff0000000000000ull;
+}
+
+// axis_coord(L, x), its product with the power of two and its truncation on
+// the integer bits where x lies in the domain
+__device__ __forceinline__ uint64_t axis_coord_bits(int L, double x)
+{
+    const double u = __dadd_rn(x, (double)kExtent / 2.0);
+    const unsigned hi = (unsigned)__double2hiint(u);
+    // 2^-512 <= u < 4
+    if (hi - 0x1ff00000u < 0x40100000u - 0x1ff00000u) {
+        const int drop = 52 - ((int)(hi >> 20) - 1023) - (L - kLevelShift);
+        const uint64_t m = ((uint64_t)__double_as_longlong(u) & 0xfffffffffffffull) | 0x10000000000000ull;
+        return (drop < 53) ? m >> drop : 0ull;
+    }
+    return axis_coord(L, x);
+}
+
+// coord_center(L, c) for c < 2^32: c + 1/2 from the bits of 2^52 + c, the rest
+// exact as there
+__device__ __forceinline__ double coord_center_bits(int L, uint64_t c)
+{
+    const double v = __dsub_rn(__hiloint2double(0x43300000, (int)(uint32_t)c), 4503599627370495.5);
+    return __dadd_rn(times_pow2(v, kLevelShift - L), -(double)kExtent / 2.0);
+}
+
+// a / b for a divisor with y = 1 / b rounded to nearest, correctly rounded
+// where nothing over- or underflows (Markstein, IBM J. Res. Dev. 34, 1990: a
+// quotient within one ulp and the residual of a fused multiply-add)
+__device__ __forceinline__ double divide_by(double a, double b, double y)
+{
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
 
 }  // namespace mpf

@@ -79,21 +79,6 @@ __device__ __forceinline__ double axis_factor(int scheme, int L, float x, uint64
     return __dsub_rn(0.75, __dmul_rn(dist, dist));
 }
 
-// axis_coord(L, x), its product with the power of two and its truncation on
-// the integer bits where x lies in the domain
-__device__ __forceinline__ uint64_t axis_coord_bits(int L, double x)
-{
-    const double u = __dadd_rn(x, (double)kExtent / 2.0);
-    const unsigned hi = (unsigned)__double2hiint(u);
-    // 2^-512 <= u < 4
-    if (hi - 0x1ff00000u < 0x40100000u - 0x1ff00000u) {
-        const int drop = 52 - ((int)(hi >> 20) - 1023) - (L - kLevelShift);
-        const uint64_t m = ((uint64_t)__double_as_longlong(u) & 0xfffffffffffffull) | 0x10000000000000ull;
-        return (drop < 53) ? m >> drop : 0ull;
-    }
-    return axis_coord(L, x);
-}
-
 // pairs per particle: pass 0 counts them (cnt[i]) and writes the particle's
 // axis factors per level (axw[(i * nlev + level - lmin) * 9 + 3 * axis +
 // offset + 1]); pass 1 writes the pairs at off[i] as (cell, particle << 5 |

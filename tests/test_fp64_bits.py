@@ -30,6 +30,10 @@ inline double __hiloint2double(int h, int l)
     return __longlong_as_double((long long)(((unsigned long long)(unsigned)h << 32) | (unsigned)l));
 }
 inline float __double2float_rn(double v) { return (float)v; }
+inline double __dadd_rn(double a, double b) { return a + b; }
+inline double __dsub_rn(double a, double b) { return a - b; }
+inline double __dmul_rn(double a, double b) { return a * b; }
+inline double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
 """
 
 SOURCE = r"""
@@ -43,6 +47,9 @@ EACH(t_round32, double, double, round32(a[i]), (double)(float)a[i])
 EACH(t_times_pow2, double, double, times_pow2(a[i], (int)b[i]), std::ldexp(a[i], (int)b[i]))
 EACH(t_less64, double, int, less64(a[i], b[i]), a[i] < b[i])
 EACH(t_negative, double, int, negative(a[i]), a[i] < 0.0)
+EACH(t_axis, double, unsigned long long, axis_coord_bits((int)b[i], a[i]), axis_coord((int)b[i], a[i]))
+EACH(t_center, double, double, coord_center_bits((int)b[i], (uint64_t)a[i]), coord_center((int)b[i], (uint64_t)a[i]))
+EACH(t_divide, double, double, divide_by(a[i], b[i], 1.0 / b[i]), a[i] / b[i])
 """
 
 
@@ -111,3 +118,27 @@ def test_compares(bits):
         ok = (other != 0) | (d != 0)
         bits("t_less64", d[ok], other[ok], out=np.int32)
         bits("t_less64", other[ok], d[ok], out=np.int32)
+
+
+@pytest.mark.parametrize("level", [0, 1, 2, 3, 9, 20, 31, 32])
+def test_coordinates(bits, level):
+    rng = np.random.default_rng(level)
+    cells = np.arange(-6, 7) * 2.0 ** (2 - level)
+    x = np.concatenate([rng.uniform(-2, 2, 1 << 16), rng.uniform(-6, 6, 1 << 12), cells - 2, cells, 2 + cells,
+                        [-2.0, 2.0, 0.0, -0.0, 1e-300, -1e-300, 1e9, -1e9, -np.inf, np.nan, -np.nan]])
+    x = np.concatenate([x, np.nextafter(x, np.inf), np.nextafter(x, -np.inf)])
+    x = x[~(x > 1e9)]
+    lv = np.full(x.shape, float(level))
+    bits("t_axis", x, lv, out=np.uint64)
+    c = np.unique(np.concatenate([[0, 1, 2 ** level - 1], rng.integers(0, 2 ** level, 1 << 12)])).astype(np.float64)
+    bits("t_center", c, np.full(c.shape, float(level)))
+
+
+def test_quotients_by_a_rounded_reciprocal(bits):
+    """Operands whose quotient, reciprocal and residuals stay in the normal range: box lengths and k components."""
+    rng = np.random.default_rng(5)
+    b = np.concatenate([10.0 ** rng.uniform(20, 30, 1 << 17), np.ldexp(1.0, np.arange(60, 100)), [9.293e25, 9.3e25]])
+    a = rng.choice([-1, 1], b.shape) * 10.0 ** rng.uniform(-30, 12, b.shape)
+    bits("t_divide", a, b)
+    bits("t_divide", np.nextafter(b, 0), b)
+    bits("t_divide", np.full(b.shape, 299792458.0), b)
