@@ -98,10 +98,16 @@ __global__ void k_dep_pairs(DevTree T, int scheme, int lmin, int lmax, const flo
     const long long base = off ? off[i] : 0;
     uint64_t c32[3];
     for (int d = 0; d < 3; ++d) c32[d] = axis_coord_bits(kMaxLevel, (double)p[d]);
+    // 2^34 and more from the octree's lower face, the level-32 coordinate
+    // saturates where a coarser level's still wraps: each level on its own
+    const float far = 8589934592.f;
+    const bool saturates = !(p[0] < far && p[1] < far && p[2] < far);
     int own = -1;   // the particle's cell of level L, or -1
     for (int L = lmin; L <= lmax; ++L) {
-        const uint64_t cc[3] = {c32[0] >> (kMaxLevel - L), c32[1] >> (kMaxLevel - L), c32[2] >> (kMaxLevel - L)};
-        if (L == lmin) {
+        uint64_t cc[3] = {c32[0] >> (kMaxLevel - L), c32[1] >> (kMaxLevel - L), c32[2] >> (kMaxLevel - L)};
+        if (saturates) {
+            for (int d = 0; d < 3; ++d) cc[d] = axis_coord(L, (double)p[d]);
+        } else if (L == lmin) {
             const Found f = find_cell(T, L, cc[0], cc[1], cc[2]);
             own = (f.cell >= 0 && f.level == L) ? f.cell : -1;
         } else if (own >= 0) {

@@ -195,6 +195,29 @@ def test_deposit_matches_oracle_at_tile_edges(gpu_lib, pkg, oracle_mod, synth, a
     np.testing.assert_array_equal(v.view(np.uint32), np.asarray(ov, dtype=np.float32).view(np.uint32))
 
 
+@pytest.mark.parametrize("scheme", ["cic", "tsc"])
+def test_deposit_of_particles_outside_the_octree(gpu_lib, pkg, oracle_mod, synth, amr, scheme):
+    """Particles with one coordinate outside the domain, where integer
+    coordinates wrap, and from 2^34 on saturate level by level: the C oracle's
+    bits.  (Products of two such weights would overflow a float.)"""
+    out = [2.0, 2.5, 5.99, 1e3, 3e9, 2.0 ** 33, 2.0 ** 34, 2.0 ** 36, 1e12, 1e15, -2.0, -2.5, -1e12]
+    pos, pv = synth.velocity_particles(amr["records"], 3 * 64 * len(out), seed=3)
+    for k, x in enumerate(out):
+        for d in range(3):
+            i = 64 * (3 * k + d)
+            pos[i:i + 64, d] = np.float32(x)
+    tree = pkg.Octree.from_records(amr["records"])
+    tree.deposit_velocity(pos, pv, scheme)
+    v, rho = tree.velocity()
+    tree.close()
+    O = oracle_mod.Oracle(amr["records"], {"t": amr["cosmo_t"], "a": amr["cosmo_a"], "dadt": amr["cosmo_dadt"]},
+                          float(amr["cosmo_length"]))
+    ov, orho = O.deposit_velocity(pos, pv, scheme)
+    assert np.count_nonzero(orho) > 100
+    np.testing.assert_array_equal(rho.view(np.uint32), np.asarray(orho, dtype=np.float32).view(np.uint32))
+    np.testing.assert_array_equal(v.view(np.uint32), np.asarray(ov, dtype=np.float32).view(np.uint32))
+
+
 @pytest.mark.parametrize("order", [1, 2])
 @pytest.mark.parametrize("velocity", [True, False])
 def test_redshift_tests_at_the_threshold(gpu_lib, pkg, synth, amr, vel, cosmo, order, velocity):
