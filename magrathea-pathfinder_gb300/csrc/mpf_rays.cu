@@ -257,8 +257,15 @@ extern "C" int mpf_rays_propagate(const mpf_octree* o, const mpf_cosmology* c, c
     if (e == cudaSuccess) e = dsizes.alloc((size_t)chunk * sizeof(long long));
     if (e == cudaSuccess) e = dstatus.alloc(sizeof(unsigned));
     if (e != cudaSuccess) return cuda_fail(e, "mpf_rays_propagate");
-    std::vector<double> launch((size_t)chunk * nt * 6), dirs((size_t)nt * 3), points;
-    std::vector<long long> steps((size_t)chunk * nt);
+    std::vector<double> launch, dirs, points;
+    std::vector<long long> steps;
+    try {
+        launch.resize((size_t)chunk * nt * 6);
+        dirs.resize((size_t)nt * 3);
+        steps.resize((size_t)chunk * nt);
+    } catch (const std::bad_alloc&) {
+        return fail(MPF_OUT_OF_MEMORY, "mpf_rays_propagate: no host memory for the launch records");
+    }
     int rc = MPF_OK;
     for (long long b0 = 0; b0 < n; b0 += chunk) {
         const long long m = std::min<long long>(chunk, n - b0);
