@@ -873,7 +873,10 @@ def main():
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": (DRAM_BYTES_PER_PHOTON_STEP * photon_steps / args.steps) if DRAM_BYTES_PER_PHOTON_STEP else None,
                 "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
-                "bytes_per_photon_step": BYTES_PER_PHOTON_STEP}
+                "bytes_per_photon_step": BYTES_PER_PHOTON_STEP,
+                "note": "achieved counts the payload bytes the algorithm requests, which L1 and L2 serve (DRAM moves "
+                        "traffic bytes a launch): a rate, not a distance to a floor; the kernel is bound by the latency "
+                        "of two warps a scheduler and the FP64 pipe"}
     clk_summary = clk.summary()
     roofline["fp64"] = fp64_roofline(value / world, clk_summary)
     tuned = pkg.autotune_info(tree, "propagate", 2)

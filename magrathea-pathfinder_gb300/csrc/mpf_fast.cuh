@@ -1,6 +1,6 @@
 // Throughput mode of the propagation kernel.
 //
-// Same algorithm as propagate_one<EXACT> (src/integrator.h:648-824 with the
+// Same algorithm as propagate_one (mpf_exact.cuh: src/integrator.h:648-824 with the
 // fused src/lensing.h:399-472 Jacobian), reorganised for the GB300's
 // arithmetic balance:
 //
@@ -481,7 +481,6 @@ __device__ __forceinline__ Field7 gather_at(const DevTree& T, const Spot& d, con
 struct FastRec {
     double a, t, x, y, z, k0, k1, k2, k3;
     double phi, red, chi, lambda, s, isw, iswold;
-    double dop;   // velocity-field octrees: the point's Doppler term v.k / (c k0)
     float rho, dx, dy, dz, dt, ah;   // dt: the photon's (forward) dphidt
     int level;
 };
@@ -858,8 +857,7 @@ struct RaySlots {
 // The lanes that trace one ray: a full warp has one ray a lane; a warp with
 // few rays gives each of them 2, 3 or 6 lanes, which take the same steps with
 // the same values (and write the same outputs) and share out the six gathers
-// of the Jacobian, the larger part of a step.
-__host__ __device__ __forceinline__ int rays_to_lanes(int rays) { return (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1; }
+// of the Jacobian, the larger part of a step (rays_to_lanes).
 struct RayLanes {
     int per_ray;     // 1, 2, 3 or 6
     int sub;         // this lane's place among them
@@ -1004,6 +1002,11 @@ __device__ void propagate_fast(const DevTree& T, const DevCosmo& C, const PropPa
     // velocity field 3.53 -> 3.35.  A plain TSC step with the Jacobian's six
     // gathers (2 200 instructions) waits for instructions as much as for that
     // pipe, and the added code made it slower (60 000 map rays 119 -> 126 ms).
+    // The order decides, not the Jacobian, which no instantiation knows: CIC
+    // with it still gains (20 011 rays on a uniform cone 6.40 -> 6.16 ms,
+    // 3 001 and 60 000 on a refined one 30.7 -> 29.6 and 111 -> 109), and TSC
+    // without it hardly (bundle maps of 9 001 pixels 35.6 -> 35.2 ms, 20 011
+    // plain rays 35.1 in both forms).
     constexpr bool kLean = ORDER == 1 || VEL;
     // Stage 1 written out, the table slope kept for the step and the surface
     // record out of line pay everywhere but in the TSC source instantiation,

@@ -41,7 +41,7 @@ cudaError_t launch_propagate<true>(const DevTree& T, const DevCosmo& C, const Pr
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const int rays = (int)std::min<long long>(32, (n + 4 * sms - 1) / (4 * sms));
-    const int per_ray = !P.jacobian ? 1 : (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1;
+    const int per_ray = P.jacobian ? rays_to_lanes(rays) : 1;
     const long long warps = (n + rays - 1) / rays;
     const int tpb = (warps < 8ll * sms) ? 32 : 128;
     const unsigned grid = (unsigned)((warps + tpb / 32 - 1) / (tpb / 32));

@@ -90,11 +90,12 @@ static FastShape fast_launch_shape(long long n, int blocks_per_sm, int sms, bool
 
 // ---------------------------------------------------------------------------
 // Order of a batch's rays on a refined octree: by the Morton index of their
-// direction on a 128 x 128 grid over the directions' own bounding box.  The rays of a warp then
-// read the same stencils, and the warps at work at one time the same cells,
-// whatever the caller's order: 160 000 rays to z = 2 on a refined cone 433 ->
-// 408 ms from rows of a pixel grid and 736 -> 408 ms from a shuffled list;
-// 60 000 137 -> 125 and 210 -> 125 ms.  Rays in one square of the grid come
+// direction on a 128 x 128 grid over the directions' own bounding box.  The
+// rays of a warp then read the same stencils, and the warps at work at one time
+// the same cells, whatever the caller's order: 160 000 rays to z = 2 on a
+// refined cone 432 -> 393 ms from rows of a pixel grid and 709 -> 394 ms from a
+// shuffled list, 60 000 204 -> 188 and 290 -> 188, 20 011 103 -> 97 and 124 ->
+// 98; the maps of 60 000 pixels to z = 1 138 -> 118.  Rays in one square of the grid come
 // in any order; a ray's result does not depend on it.  Below kOrderMinRays the
 // five launches (25 us) cost more than they give; on an octree of one level,
 // where the rays of a warp hardly diverge, rows measured 6 % faster than the

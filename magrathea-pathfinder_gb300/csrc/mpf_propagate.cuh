@@ -135,4 +135,8 @@ __device__ __forceinline__ void write_rec(double* o, const Rec& r)
 
 constexpr double kC = 299792458.0;
 
+// The lanes of a warp that trace one ray together when it has `rays` of them
+// and a Jacobian, whose six gathers they share out.
+__host__ __device__ __forceinline__ int rays_to_lanes(int rays) { return (rays <= 5) ? 6 : (rays <= 10) ? 3 : (rays <= 16) ? 2 : 1; }
+
 }  // namespace mpf
