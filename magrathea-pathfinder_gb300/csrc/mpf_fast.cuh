@@ -280,7 +280,7 @@ __device__ __forceinline__ Loc locate_rel(const DevTree& T, const Loc& h, float 
             r.f[0] = rx; r.f[1] = ry; r.f[2] = rz;
             return r;
         }
-        if (abs(ox) <= 1 && abs(oy) <= 1 && abs(oz) <= 1) {
+        if (within_one_cell(ox, oy, oz)) {
             const int e = rec_entry(T, h.cell, (ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
             if (e >= 0) {
                 const int fl = rec_flags(T, e);
@@ -631,7 +631,7 @@ __device__ __forceinline__ int find_spot(const DevTree& T, const Spot& h, int ox
     d.f[0] = fx; d.f[1] = fy; d.f[2] = fz;
     const bool same = h.cell >= 0 && (ox | oy | oz) == 0;
     int q = same ? h.cell : -1, kind = same ? kSpotSame : kSpotLeaf;
-    if (!same && h.cell >= 0 && abs(ox) <= 1 && abs(oy) <= 1 && abs(oz) <= 1)
+    if (!same && h.cell >= 0 && within_one_cell(ox, oy, oz))
         q = rec_entry(T, h.cell, (ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
     if (q >= 0) {
         r7 = __ldg(T.stencil + 8 * (size_t)q + 7);

@@ -57,6 +57,13 @@ MPF_HD uint64_t axis_coord(int level, double x)
     return (level >= 64) ? c : (c & ((1ull << level) - 1ull));
 }
 
+// Offsets of -1, 0 or 1 cell along every axis: a place in a cell's stencil
+// record.  (abs(o) <= 1 holds for INT_MIN, the conversion of an offset far below.)
+MPF_HD bool within_one_cell(int ox, int oy, int oz)
+{
+    return (unsigned)ox + 1u <= 2u && (unsigned)oy + 1u <= 2u && (unsigned)oz + 1u <= 2u;
+}
+
 // Key of the level-`level` cell with integer coordinates (cx, cy, cz).
 MPF_HD Key key_from_coords(int level, uint64_t cx, uint64_t cy, uint64_t cz)
 {
