@@ -225,6 +225,44 @@ __device__ __forceinline__ double tsc_w1(int a, double d)
     return __dsub_rn(0.75, __dmul_rn(d, d));
 }
 
+// tsc_exact at a point with a level-32 coordinate of all ones: it may have
+// saturated (from 2^34 on) where a coarser level's still wraps, so every
+// vertex's coordinates are formed at its own level.  Out of line: rays do not
+// get there.
+template <int F, bool V>
+static __device__ __noinline__ Field7 tsc_saturated(const DevTree& T, double x, double y, double z, Hint& hint, float* vv)
+{
+    ExactAcc<F, V> res;
+    res.reset();
+    const uint64_t c32[3] = {axis_coord(kMaxLevel, x), axis_coord(kMaxLevel, y), axis_coord(kMaxLevel, z)};
+    const Found f0 = locate_near32(T, c32, hint);
+    if (f0.cell < 0) return res.field(vv);
+    int ilvl = f0.level, lvl = ilvl;
+    const double pt[3] = {x, y, z};
+    do {
+        ilvl = lvl;
+        const double tw = cell_extent(ilvl);
+        bool stop = false;
+#pragma unroll 1
+        for (int v = 0; v < 27 && !stop; ++v) {
+            double w = 1.0;
+            uint64_t k[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int o = (d == 0 ? v / 9 : d == 1 ? (v / 3) % 3 : v % 3) - 1;
+                k[d] = axis_coord(ilvl, __dadd_rn(pt[d], o == 0 ? 0.0 : o > 0 ? tw : -tw));
+                w = __dmul_rn(w, tsc_w1(o != 0, fabs(times_pow2(__dsub_rn(coord_center(ilvl, k[d]), pt[d]), ilvl - kLevelShift))));
+            }
+            const Found fi = find_cell(T, ilvl, k[0], k[1], k[2]);
+            if (fi.cell >= 0) lvl = min(lvl, fi.level);
+            stop = fi.cell < 0 || lvl < ilvl;
+            if (!stop) res.add(T, fi.cell, w);
+        }
+        if (stop) res.reset();
+    } while (lvl < ilvl);
+    return res.field(vv);
+}
+
 // Triangular-shaped cloud (simplehyperoctree.h:1479-1644): quadratic weights
 // over the 27 cells of the located cell's level, x-major (ix, iy, iz) order;
 // restarts at the level of the first coarser neighbour; empty when one is
@@ -236,6 +274,10 @@ __device__ Field7 tsc_exact(const DevTree& T, double x, double y, double z, Hint
     ExactAcc<F, V> res;
     res.reset();
     const uint64_t c32[3] = {axis_coord_bits(kMaxLevel, x), axis_coord_bits(kMaxLevel, y), axis_coord_bits(kMaxLevel, z)};
+    // (the stages and the Jacobian's points of a ray lie within a step and a cell
+    // of the domain, those of other rays are not kept)
+    const uint64_t ones = 0xffffffffull;
+    if (F == kAllFields && (c32[0] == ones || c32[1] == ones || c32[2] == ones)) return tsc_saturated<F, V>(T, x, y, z, hint, vv);
     const Found f0 = locate_near32(T, c32, hint);
     if (f0.cell < 0) return res.field(vv);
     int ilvl = f0.level, lvl = ilvl;
